@@ -282,10 +282,18 @@ cudaError_t fork_side(dns3d_handle* h, int i) {
     return e ? e : cudaStreamWaitEvent(h->side, h->fork_ev[i], 0);
 }
 
+// the two halves of the join: where the side work it covers ends (later side
+// work is not waited for), and where the handle's stream needs it
+cudaError_t record_join(dns3d_handle* h, int i) {
+    return h->prof ? cudaSuccess : cudaEventRecord(h->join_ev[i], h->side);
+}
+cudaError_t wait_join(dns3d_handle* h, int i) {
+    return h->prof ? cudaSuccess : cudaStreamWaitEvent(h->stream, h->join_ev[i], 0);
+}
+
 cudaError_t join_side(dns3d_handle* h, int i) {
-    if (h->prof) return cudaSuccess;
-    cudaError_t e = cudaEventRecord(h->join_ev[i], h->side);
-    return e ? e : cudaStreamWaitEvent(h->stream, h->join_ev[i], 0);
+    const cudaError_t e = record_join(h, i);
+    return e ? e : wait_join(h, i);
 }
 
 // Parity folding of a full row-major operator (see step.cu): antisymmetric
@@ -348,6 +356,19 @@ int run_source_terms_mixed(dns3d_handle* h, double2* const* in) {
     const GridDev& g = h->g;
     FFields sp{};
     for (int f = 0; f < 6; ++f) sp.p[f] = h->spec32[f];
+    if (h->fft.use_ct) {
+        // one y pass of all six fields, u, v, w as the vorticity kernel rounded
+        // them (batches read the FP64 state in a y pass of its own beside the
+        // vorticity, the same values: alone that was 196 us per step against
+        // 189 at 128x128x65, 73 against 67 at 64x48x40)
+        FFields src{};
+        for (int f = 0; f < 3; ++f) src.p[f] = h->src32[f];
+        CK(h, launch_vorticity_mixed(g, h->mx, h->ops, in[0], in[1], in[2], sp, h->stream));
+        mark(h, "vorticity32");
+        // the 2/3 filter discards kx > kx_max: those columns are not completed
+        CK(h, nl_transforms32(h->fft, g, sp, src, h->sp.dealias ? h->sp.kx_max + 1 : 0, h->stream));
+        return DNS3D_OK;
+    }
     CK(h, launch_vorticity_mixed(g, h->mx, h->ops, in[0], in[1], in[2], sp, h->stream));
     mark(h, "vorticity32");
     FRFields ph{};
@@ -420,7 +441,9 @@ int run_source_terms_fp64(dns3d_handle* h, double2* const* in) {
             su.p[f] = in[f];
             pu.p[f] = h->phys[f];
         }
-        CK(h, fft_c2r(h->fft, g, su, pu, 3, g.nz, side_stream(h), 0));
+        if (h->fft.fx) CK(h, nl_y_inverse(h->fft, g, su, 3, 0, side_stream(h)));
+        else CK(h, fft_c2r(h->fft, g, su, pu, 3, g.nz, side_stream(h), 0));
+        CK(h, record_join(h, 1));
     }
     // vorticity into the u*,v*,w* buffers (free until the viscous step)
     if (h->vort_tc) {
@@ -432,20 +455,27 @@ int run_source_terms_fp64(dns3d_handle* h, double2* const* in) {
     }
     Fields spec{};
     spec.p[0] = h->US; spec.p[1] = h->VS; spec.p[2] = h->WS;
+    Fields src{};
+    src.p[0] = h->SU; src.p[1] = h->SV; src.p[2] = h->SW;
+    // the 2/3 filter discards kx > kx_max: those columns are not completed
+    const int ncol = h->sp.dealias ? h->sp.kx_max + 1 : 0;
+    if (h->fft.fx) {
+        CK(h, nl_y_inverse(h->fft, g, spec, 3, 3, h->stream));
+        CK(h, wait_join(h, 1));
+        CK(h, nl_products(h->fft, g, src, ncol, h->stream));
+        return DNS3D_OK;
+    }
     RFields phys{};
     for (int f = 0; f < 3; ++f) phys.p[f] = h->phys[3 + f];
     CK(h, fft_c2r(h->fft, g, spec, phys, 3, g.nz, h->stream, 3));
-    CK(h, join_side(h, 1));
+    CK(h, wait_join(h, 1));
     RFields all{};  // u, v, w, ox, oy, oz in physical space
     for (int f = 0; f < 6; ++f) all.p[f] = h->phys[f];
     RFields prod{};
     for (int f = 0; f < 3; ++f) prod.p[f] = h->phys[f];
     CK(h, launch_products(g, all, prod, h->stream));
     mark(h, "products");
-    Fields src{};
-    src.p[0] = h->SU; src.p[1] = h->SV; src.p[2] = h->SW;
-    // the 2/3 filter discards kx > kx_max: those columns skip the y pass
-    CK(h, fft_r2c(h->fft, g, prod, src, 3, g.nz, h->stream, h->sp.dealias ? h->sp.kx_max + 1 : 0));
+    CK(h, fft_r2c(h->fft, g, prod, src, 3, g.nz, h->stream, ncol));
     return DNS3D_OK;
 }
 
@@ -638,8 +668,15 @@ int dns3d_footprint_bytes(const dns3d_config* c, unsigned long long* bytes) {
     const size_t hz = (size_t)c->nz / 2, ez = (size_t)c->nz - hz;
     b += (2 * nq * (ez * ez + hz * hz) + 2 * nz2) * sizeof(double);  // folded inverses, pinned, S
     if (c->precision == DNS3D_PREC_MIXED)
-        b += (6 + 3 + 6) * se * sizeof(float2) + 6 * pe * sizeof(float) + se * sizeof(double2);  // + dphi/dz
-    else if (tc_supported(c->nz)) {
+        // FP32 spectra, sources and scratch, dphi/dz (and the physical planes
+        // without compile-time transforms)
+        b += (6 + 3 + 6) * se * sizeof(float2) + se * sizeof(double2) +
+             (fft_ct_supported(c->ny, c->nx / 2) ? 0 : 6 * pe * sizeof(float));
+    else {
+        if (fft_ct_supported(c->ny, c->nx / 2))  // exponents of the nonlinear term's integer spectra
+            b += ((size_t)6 * (c->nx / 2 + 1) + (size_t)3 * c->ny) * c->nz * sizeof(int);
+    }
+    if (c->precision != DNS3D_PREC_MIXED && tc_supported(c->nz)) {
         const TcGeom t = tc_geom(c->nz);
         if (c->use_crank_nicolson && c->linear_solver == 0)  // digit slices of the Helmholtz inverses
             b += nq * (tc_q_halves(t) * sizeof(__half) + (size_t)t.m8 * sizeof(int));
@@ -1007,6 +1044,10 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
 
     cudaError_t e;
     if ((e = fft_setup(h->fft, g)) != cudaSuccess) { cuda_fail(h, e, "fft_setup"); return fail(DNS3D_E_CUDA); }
+    if (h->fft.fx && c.precision != DNS3D_PREC_MIXED &&
+        ((rc = dev_alloc(h, &h->fft.ecol, (size_t)6 * nz * g.nxhp)) ||
+         (rc = dev_alloc(h, &h->fft.erow, (size_t)3 * nz * c.ny))))
+        return fail(rc);
     if ((e = prepare_step_kernels(g)) != cudaSuccess) { cuda_fail(h, e, "prepare"); return fail(DNS3D_E_CUDA); }
 
     // per-mode operator inverses
@@ -1216,8 +1257,11 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
             {mx.Se_df, Se_df.data(), Se_df.size() * 8}, {mx.So_df, So_df.data(), So_df.size() * 8}};
         for (auto& u : u32)
             if ((rc = upload(h, u.d, u.s, u.b))) return fail(rc);
-        for (int f = 0; f < 6; ++f)
-            if ((rc = dev_alloc(h, &h->spec32[f], se)) || (rc = dev_alloc(h, &h->phys32[f], pe))) return fail(rc);
+        for (int f = 0; f < 6; ++f) {
+            if ((rc = dev_alloc(h, &h->spec32[f], se))) return fail(rc);
+            // with compile-time transforms the physical planes stay on the SM
+            if (!h->fft.use_ct && (rc = dev_alloc(h, &h->phys32[f], pe))) return fail(rc);
+        }
         for (int f = 0; f < 3; ++f)
             if ((rc = dev_alloc(h, &h->src32[f], se))) return fail(rc);
         if ((rc = dev_alloc(h, &h->fft.tmp32, 6 * se))) return fail(rc);
@@ -1999,7 +2043,7 @@ int dns3d_lgl_nodes_weights(int nz, double* z, double* w) {
 // ------------------------------------------------------------------ batches
 // Joint stepping of independent runs.  Eligible runs of one precision and one
 // kernel variant (which stages run their tensor-core bodies) form a group
-// whose step is ten ragged stage launches (ragged.cuh): a group's launch sizes
+// whose step is a sequence of ragged stage launches (ragged.cuh): a group's launch sizes
 // its shared memory for its largest run, so runs of different variants are not
 // mixed.  The others keep their own step bodies; every group and loose run is
 // a branch of the same graph.
@@ -2010,6 +2054,7 @@ struct dns3d_batch {
         int variant = 0;              // RaggedVariant bits (FP64 groups)
         cudaStream_t lane = nullptr, side = nullptr;  // side: the mixed form's mode (0,0) stages
         cudaEvent_t lane_join = nullptr, side_fork = nullptr, side_join = nullptr;
+        cudaEvent_t uvw_fork = nullptr, uvw_join = nullptr, pi_join = nullptr;
         std::vector<int> idx;         // runs of the group (indices into runs)
         std::vector<RunDesc> desc;    // host copies of the descriptors
         std::vector<int> own_tc;      // per run, the tile widths of its own launches [kTileKernels]
@@ -2095,7 +2140,7 @@ RunDesc make_desc(const dns3d_handle* h) {
     const size_t se = spec_elems(h->cfg);
     if (h->mixed) {
         for (int f = 0; f < 6; ++f) {
-            d.spec[f] = h->spec32[f];
+            d.spec[f] = f < 3 ? static_cast<void*>(f == 0 ? h->U : f == 1 ? h->V : h->W) : h->spec32[f];
             d.tmp[f] = h->fft.tmp32 + (size_t)f * se;
             d.phys[f] = h->phys32[f];
         }
@@ -2112,6 +2157,7 @@ RunDesc make_desc(const dns3d_handle* h) {
         d.fftfx = h->fft.fx ? 1 : 0;
         if (d.fftfx) {
             d.tw_ny = h->fft.twq_ny; d.tw_nx2 = h->fft.twq_nx2; d.tw_nx = h->fft.twq_nx;
+            d.ecol = h->fft.ecol; d.erow = h->fft.erow; d.nl = h->fft.nl;
         } else {
             d.tw_ny = h->fft.tw_ny; d.tw_nx2 = h->fft.tw_nx2; d.tw_nx = h->fft.tw_nx;
         }
@@ -2173,14 +2219,12 @@ cudaError_t group_launch(dns3d_batch::Group& G, int s, cudaStream_t st) {
     RunDesc* runs = G.d_desc;
     void* args[] = {&runs, &map};
     return cudaLaunchKernel((const void*)ragged_kernel(s, G.mixed, G.variant), dim3((unsigned)G.total[s]),
-                            dim3(kStageThreads), args, G.smem[s], st);
+                            dim3((unsigned)ragged_threads(s)), args, G.smem[s], st);
 }
 
 // Stage tile widths for the group: each run's own widths, or one width for
 // all runs, whichever launch is fastest (one warm launch, then three between
-// events).  The stages timed write only work buffers, apart from the PI
-// update in front of the vorticity tiles, whose controller states the caller
-// restores.
+// events).  The stages timed write only work buffers.
 int group_tune(dns3d_batch* b, dns3d_batch::Group& G) {
     const int n = (int)G.idx.size();
     cudaEvent_t e0, e1;
@@ -2232,7 +2276,7 @@ void batch_release(dns3d_batch* b) {
     for (auto& G : b->grp) {
         cudaFree(G.d_desc);
         cudaFree(G.d_map);
-        for (auto ev : {G.lane_join, G.side_fork, G.side_join})
+        for (auto ev : {G.lane_join, G.side_fork, G.side_join, G.uvw_fork, G.uvw_join, G.pi_join})
             if (ev) cudaEventDestroy(ev);
         for (auto st : {G.lane, G.side})
             if (st) cudaStreamDestroy(st);
@@ -2244,7 +2288,8 @@ void batch_release(dns3d_batch* b) {
     if (b->stream) cudaStreamDestroy(b->stream);
 }
 
-// One group's step on its lane: the nonlinear-term stages, then viscous and
+// One group's step on its lane: the nonlinear-term stages (the state's inverse
+// y pass and the PI update on a forked stream), then viscous and
 // pressure tiles with (mixed form) the mode (0,0) chain forked beside them,
 // then projection and walls.
 cudaError_t group_capture(dns3d_batch::Group& G, int* launches) {
@@ -2256,8 +2301,19 @@ cudaError_t group_capture(dns3d_batch::Group& G, int* launches) {
             *launches += 1;
         }
     };
-    for (int s : {(int)kRsVort, (int)kRsFftYInv, (int)kRsFftC2R, (int)kRsProd, (int)kRsFftR2C, (int)kRsFftYFwd})
-        stage(s, lane);
+    // beside the vorticity: the state's inverse y pass (the x stages wait for
+    // it) and the PI update (the viscous stages wait for it)
+    ce = cudaEventRecord(G.uvw_fork, lane);
+    if (!ce) ce = cudaStreamWaitEvent(side, G.uvw_fork, 0);
+    stage(kRsFftYUvw, side);
+    if (!ce) ce = cudaEventRecord(G.uvw_join, side);
+    stage(kRsPi, side);
+    if (!ce) ce = cudaEventRecord(G.pi_join, side);
+    stage(kRsVort, lane);
+    stage(kRsFftYInv, lane);
+    if (!ce) ce = cudaStreamWaitEvent(lane, G.uvw_join, 0);
+    for (int s : {(int)kRsFftX, (int)kRsFftC2R, (int)kRsProd, (int)kRsFftR2C, (int)kRsFftYFwd}) stage(s, lane);
+    if (!ce) ce = cudaStreamWaitEvent(lane, G.pi_join, 0);
     if (G.mixed) {
         if (!ce) ce = cudaEventRecord(G.side_fork, lane);
         if (!ce) ce = cudaStreamWaitEvent(side, G.side_fork, 0);
@@ -2379,6 +2435,9 @@ int batch_create(dns3d_handle* const* runs, int nruns, int flags, dns3d_batch** 
         if (cudaStreamCreateWithFlags(&G.lane, cudaStreamNonBlocking) ||
             cudaStreamCreateWithFlags(&G.side, cudaStreamNonBlocking) ||
             cudaEventCreateWithFlags(&G.lane_join, cudaEventDisableTiming) ||
+            cudaEventCreateWithFlags(&G.uvw_fork, cudaEventDisableTiming) ||
+            cudaEventCreateWithFlags(&G.uvw_join, cudaEventDisableTiming) ||
+            cudaEventCreateWithFlags(&G.pi_join, cudaEventDisableTiming) ||
             cudaEventCreateWithFlags(&G.side_fork, cudaEventDisableTiming) ||
             cudaEventCreateWithFlags(&G.side_join, cudaEventDisableTiming))
             return fail(DNS3D_E_CUDA);
@@ -2391,13 +2450,6 @@ int batch_create(dns3d_handle* const* runs, int nruns, int flags, dns3d_batch** 
         if (cudaStreamSynchronize(runs[i]->stream)) return fail(DNS3D_E_CUDA);
     const char* env = std::getenv("DNS3D_AUTOTUNE");
     const bool tune = (flags & DNS3D_BATCH_TUNE) && !(env && std::strcmp(env, "0") == 0);
-    std::vector<dns3d_pi_state> pis;
-    if (tune) {
-        pis.resize(nruns);
-        for (int i = 0; i < nruns; ++i)
-            if (cudaMemcpy(&pis[i], runs[i]->d_pi, sizeof(dns3d_pi_state), cudaMemcpyDeviceToHost))
-                return fail(DNS3D_E_CUDA);
-    }
     for (auto& G : b->grp) {
         if (G.idx.empty()) continue;
         rc = tune ? group_tune(b, G) : group_upload(b, G);
@@ -2406,12 +2458,8 @@ int batch_create(dns3d_handle* const* runs, int nruns, int flags, dns3d_batch** 
             return fail(rc);
         }
     }
-    if (tune) {
-        for (int i = 0; i < nruns; ++i)
-            if (cudaMemcpy(runs[i]->d_pi, &pis[i], sizeof(dns3d_pi_state), cudaMemcpyHostToDevice))
-                return fail(DNS3D_E_CUDA);
+    if (tune)
         for (dns3d_handle* h : b->runs) h->phys_valid = 0;
-    }
     if ((rc = batch_capture(b))) {
         for (dns3d_handle* h : b->runs) h->err = b->err;
         return fail(rc);

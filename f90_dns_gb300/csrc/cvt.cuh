@@ -43,25 +43,23 @@ __device__ __forceinline__ float2 d2f(double2 a) { return make_float2(d2f(a.x), 
 // even), from the integer's bits: the same value as the hardware int64 -> FP64
 // conversion followed by an exact power-of-two scaling, which both issue on
 // the FP64 pipe.  Results below the normal range take that hardware path.
+// The value is normalised to its top bit first, so the rounding is one
+// add-and-carry at a fixed position for every magnitude (no branch on it).
 __device__ __forceinline__ double i2d_scaled(long long X, int e2) {
-    if (X == 0) return 0.0;
-    const unsigned long long sg = X < 0 ? 0x8000000000000000ULL : 0ULL;
+    const unsigned sg = (unsigned)((unsigned long long)X >> 32) & 0x80000000u;
     const unsigned long long a = X < 0 ? 0ULL - (unsigned long long)X : (unsigned long long)X;
-    const int p = 63 - __clzll((long long)a);  // a in [2^p, 2^(p+1))
-    const int be = p + e2 + 1023;
-    if (be <= 0) return ldexp(__ll2double_rn(X), e2);
-    unsigned long long m;
-    if (p > 52) {
-        const int sh = p - 52;
-        m = a >> sh;
-        const unsigned long long rest = a & ((1ULL << sh) - 1ULL), half = 1ULL << (sh - 1);
-        m += (rest > half || (rest == half && (m & 1ULL))) ? 1ULL : 0ULL;
-    } else {
-        m = a << (52 - p);
+    if (a == 0) return 0.0;
+    const int s = __clzll((long long)a);
+    const unsigned long long n = a << s;     // [2^63, 2^64)
+    const int be = 1086 - s + e2;            // biased exponent of 2^(63 - s + e2)
+    if ((unsigned)(be - 1) >= 2046u) {
+        if (be <= 0) return ldexp(__ll2double_rn(X), e2);
+        return __longlong_as_double((long long)(((unsigned long long)(sg | 0x7FF00000u)) << 32));
     }
-    if (be >= 2047) return __longlong_as_double((long long)(sg | 0x7FF0000000000000ULL));
+    unsigned long long m = n >> 11;  // 53 bits; the dropped 11 are rounded to nearest, ties to even
+    m += (((unsigned)n & 0x7FFu) + 0x3FFu + ((unsigned)m & 1u)) >> 11;
     // m in [2^52, 2^53]: the implicit bit (or a rounding carry) adds into the exponent field
-    return __longlong_as_double((long long)(sg | (((unsigned long long)(be - 1) << 52) + m)));
+    return __longlong_as_double((long long)(m + ((unsigned long long)((((unsigned)(be - 1)) << 20) | sg) << 32)));
 }
 
 }  // namespace dns3d

@@ -77,6 +77,12 @@ __host__ __device__ inline int mode_q(int ky, int kx, int ny, int nxhp) {
 // FFTW's semantics for non-Hermitian input: inverse c2c along y, then a 1D
 // c2r along x that ignores Im of the kx=0 and kx=nx/2 entries; output scaled
 // by 1/(nx*ny) (fftw3_dns_module.f90:127-130).
+// 1/(nx ny)^2 = m 2^(e - 63) with m an integer in [2^61, 2^62] (as limbs), or 2^e
+// where it is a power of two.
+struct NlScale {
+    long long m;
+    int e, pow2;
+};
 struct FftCtx {
     FftPlan1D py;        // length ny complex
     FftPlan1D px2;       // length nx/2 complex (packed real transform)
@@ -93,6 +99,11 @@ struct FftCtx {
     // set for grids with compile-time kernels unless DNS3D_FFT_FP64=1 keeps
     // them on the FP64 pipe
     bool fx = false;
+    // the nonlinear term's integer spectra (fft_nl.cu, fx only): exponents of
+    // the y columns [6][nz nxhp] and of the product rows [3][nz ny], and 1/(nx ny)^2
+    int* ecol = nullptr;
+    int* erow = nullptr;
+    NlScale nl{};
     double2* tmp;        // spectral scratch for nf fields
     float2* tmp32 = nullptr;  // FP32 spectral scratch (mixed path)
     int tmp_fields;
@@ -125,6 +136,17 @@ cudaError_t fft_fx_c2r_x(Fields src, RFields dst, RFields dst2, const GridDev& g
 // bulk copies)
 cudaError_t fft_fx_r2c_x(RFields src, Fields dst, const GridDev& g, int nrows, int nf, const longlong2* tw_n,
                          const longlong2* tw_nx, bool host_src, cudaStream_t s);
+
+// ---------------------------------------------------------------- fft_nl.cu
+// The transforms of the nonlinear term.  FP64 (ctx.fx): nl_y_inverse takes nf
+// spectra to the scratch slots slot0 .. slot0 + nf - 1 (slots 0-2 u, v, w, 3-5
+// the vorticity; calls on different slots can run concurrently); nl_products
+// then takes all six to the source spectra src[0..2] of u x omega (columns
+// kx < ncol, 0: all).  FP32 (ctx.use_ct): both in one call.
+cudaError_t nl_y_inverse(const FftCtx& ctx, const GridDev& g, Fields spec, int nf, int slot0, cudaStream_t s);
+cudaError_t nl_products(const FftCtx& ctx, const GridDev& g, Fields src, int ncol, cudaStream_t s);
+cudaError_t nl_transforms32(const FftCtx& ctx, const GridDev& g, FFields spec, FFields src, int ncol,
+                            cudaStream_t s);
 
 cudaError_t fft_setup(FftCtx& ctx, const GridDev& g);
 void fft_release(FftCtx& ctx);

@@ -292,14 +292,25 @@ cudaError_t smem_attr(K k, int bytes) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
 }
 
-// round(2^62 e^{-2 pi i t/n}), t < count, from the long double values.
+// A Q62 integer as two signed 32-bit limbs, w = w1 2^32 + w0 with |w0| < 2^31
+// (high word w1, low word w0), the operand form of the fixed-point products
+// (FxLimbs, fft_ct.cu).  w0 = -2^31, whose negation has no 32-bit form, is
+// stored for w + 1 instead (2^-62 off).
+long long pack_limbs(long long w) {
+    if ((int32_t)w == INT32_MIN) ++w;
+    const int32_t w0 = (int32_t)w;
+    const int64_t w1 = (w - w0) >> 32;
+    return (long long)(((uint64_t)w1 << 32) | (uint32_t)w0);
+}
+
+// round(2^62 e^{-2 pi i t/n}), t < count, from the long double values, as limbs.
 longlong2* upload_table_q62(int n, int count) {
     std::vector<longlong2> h(count);
     const long double pi = 3.141592653589793238462643383279502884L;
     for (int t = 0; t < count; ++t) {
         const long double ang = -2.0L * pi * (long double)t / (long double)n;
-        h[t].x = llroundl(ldexpl(cosl(ang), 62));
-        h[t].y = llroundl(ldexpl(sinl(ang), 62));
+        h[t].x = pack_limbs(llroundl(ldexpl(cosl(ang), 62)));
+        h[t].y = pack_limbs(llroundl(ldexpl(sinl(ang), 62)));
     }
     longlong2* d = nullptr;
     if (cudaMalloc(&d, sizeof(longlong2) * count) != cudaSuccess) return nullptr;
@@ -331,6 +342,12 @@ cudaError_t fft_setup(FftCtx& ctx, const GridDev& g) {
         ctx.twq_nx2 = upload_table_q62(g.nxh, g.nxh);
         ctx.twq_nx = upload_table_q62(g.nx, g.nxh + 1);
         if (!ctx.twq_ny || !ctx.twq_nx2 || !ctx.twq_nx) return cudaErrorMemoryAllocation;
+        const long double n = (long double)g.nx * (long double)g.ny;
+        int e = 0;
+        const long double m = frexpl(1.0L / (n * n), &e);  // [1/2, 1)
+        ctx.nl.pow2 = m == 0.5L;
+        ctx.nl.e = ctx.nl.pow2 ? e - 1 : e + 1;
+        ctx.nl.m = pack_limbs(llroundl(ldexpl(m, 62)));
     }
     const int cx = pick_cx(g.ny);
     const int rx = pick_rx(g.nxh);

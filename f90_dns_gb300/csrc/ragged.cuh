@@ -21,9 +21,12 @@ namespace dns3d {
 
 // Stages of one ragged time step, in launch order.
 enum RaggedStage {
-    kRsVort = 0,  // block 0: PI update; then vorticity mode tiles
-    kRsFftYInv,   // inverse y pass of u, v, w, ox, oy, oz
-    kRsFftC2R,    // c2r x pass of the same six fields
+    kRsVort = 0,  // vorticity mode tiles
+    kRsFftYUvw,   // inverse y pass of u, v, w, then the PI update, on a forked
+    kRsPi,        // stream beside the vorticity (they read the state only)
+    kRsFftYInv,   // inverse y pass of ox, oy, oz
+    kRsFftX,      // c2r, u x omega, r2c in one pass over the x rows (mixed, and FP64 in fixed point)
+    kRsFftC2R,    // FP64-pipe transforms instead of it: c2r x pass of the six fields
     kRsProd,      // u x omega in physical space
     kRsFftR2C,    // r2c x pass of the three products
     kRsFftYFwd,   // forward y pass of the products (2/3-filtered columns only)
@@ -51,7 +54,7 @@ struct RunDesc {
     PIParams pp;
     dns3d_pi_state* pi;
     double2 *U, *V, *W, *P, *GP, *US, *VS, *WS, *PHI, *PHIZ;
-    void* spec[6];   // c2r inputs: u, v, w, ox, oy, oz spectra (FP32 or FP64)
+    void* spec[6];   // inverse transform inputs: u, v, w (FP64), ox, oy, oz spectra (FP32 or FP64)
     void* tmp[6];    // y-pass outputs
     void* phys[6];   // physical planes; the products overwrite the first three
     void* src[3];    // nonlinear source spectra
@@ -60,6 +63,8 @@ struct RunDesc {
     const void* tw_nx;
     int* tcerr;              // tensor-core wait status of the run (viscous stage)
     int ncol;                // columns the forward y pass completes
+    int *ecol, *erow;        // fixed point: exponents of the integer spectra (FftCtx)
+    NlScale nl;
     int gx[kRsStages];       // virtual blocks per field of each stage (transforms, elementwise passes);
                              // kRsVisc: operator indices per CTA of the tensor-core viscous body
     int tcmask;              // z-derivatives on the tensor cores: 1 vorticity, 2 projection, 4 pressure
@@ -120,6 +125,10 @@ int ragged_variant(const RunDesc& d);
 // variant) or mixed runs (step.cu; the transform passes come from fft_ct.cu).
 StageKernel ragged_kernel(int stage, bool mixed, int variant);
 StageKernel ragged_fft_kernel(int stage, bool mixed, bool fx);
+StageKernel ragged_nl_kernel(int stage, bool mixed);  // fft_nl.cu
+int nl_x_threads();       // threads per CTA and x rows per CTA of kRsFftX
+int nl_x_rows(int nxh);
+int ragged_threads(int stage);
 // CTA columns (y pass) or rows (x passes) of the compile-time transform of length n.
 int fft_ct_per_cta(int n);
 // Fills d.gx for the run's grid (d.g, d.ncol set).

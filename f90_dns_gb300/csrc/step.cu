@@ -2354,9 +2354,11 @@ __device__ __forceinline__ void vorticity_mixed_body(GridDev g, MixedOps mx, Ops
             const float2 du = p ? make_float2(due.x - duo.x, due.y - duo.y) : make_float2(due.x + duo.x, due.y + duo.y);
             const float2 dv = p ? make_float2(dve.x - dvo.x, dve.y - dvo.y) : make_float2(dve.x + dvo.x, dve.y + dvo.y);
             // (i a) f = (-a f.y, a f.x)
-            out.p[0][o] = u;
-            out.p[1][o] = v;
-            out.p[2][o] = w;
+            if (out.p[0]) {  // FP32 copies of the state (the transforms without compile-time lengths)
+                out.p[0][o] = u;
+                out.p[1][o] = v;
+                out.p[2][o] = w;
+            }
             out.p[3][o] = make_float2(-ay * w.y - dv.x, ay * w.x - dv.y);          // wy - vz
             out.p[4][o] = make_float2(du.x + ax * w.y, du.y - ax * w.x);           // uz - wx
             out.p[5][o] = make_float2(-ax * v.y + ay * u.y, ax * v.x - ay * u.x);  // vx - uy
@@ -3689,14 +3691,17 @@ __device__ __forceinline__ Fields fields3(double2* a, double2* b, double2* c) {
     return f;
 }
 
+struct RsPi {
+    static constexpr int kMinCtas = 1;
+    static __device__ __forceinline__ void run(const RunDesc& d, int) {
+        pi_update_body(d.g, d.ops.zw, d.pp, d.U, d.pi, 0);
+    }
+};
+
 struct RsVort64 {
     static constexpr int kMinCtas = 2;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        if (b == 0) {
-            pi_update_body(d.g, d.ops.zw, d.pp, d.U, d.pi, 0);
-            return;
-        }
-        vorticity_body(d.g, d.ops, d.U, d.V, d.W, d.US, d.VS, d.WS, d.g.tc[kTileVort], b - 1);
+        vorticity_body(d.g, d.ops, d.U, d.V, d.W, d.US, d.VS, d.WS, d.g.tc[kTileVort], b);
     }
 };
 
@@ -3704,12 +3709,8 @@ struct RsVort64 {
 struct RsVort64Tc {
     static constexpr int kMinCtas = 1;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        if (b == 0) {
-            pi_update_body(d.g, d.ops.zw, d.pp, d.U, d.pi, 0);
-            return;
-        }
         const int ntiles = (d.g.nm + kTcVortModes - 1) / kTcVortModes, chunk = d.vort_chunk;
-        const int t0 = (b - 1) * chunk;
+        const int t0 = b * chunk;
         const VortTcOp op{d.U, d.V, d.W, d.US, d.VS, d.WS};
         dz_tc_body(d.g, d.ops, op, t0, min(t0 + chunk, ntiles), d.tcerr);
     }
@@ -3718,24 +3719,17 @@ struct RsVort64Tc {
 struct RsVort32 {
     static constexpr int kMinCtas = 4;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        if (b == 0) {
-            pi_update_body(d.g, d.ops.zw, d.pp, d.U, d.pi, 0);
-            return;
-        }
-        vorticity_mixed_body(d.g, d.mx, d.ops, d.U, d.V, d.W, desc_fields<float2, 6>(d.spec), d.g.tc[kTileVortM],
-                             b - 1);
+        FFields out = desc_fields<float2, 6>(d.spec);
+        out.p[0] = out.p[1] = out.p[2] = nullptr;  // the y pass reads the FP64 state itself
+        vorticity_mixed_body(d.g, d.mx, d.ops, d.U, d.V, d.W, out, d.g.tc[kTileVortM], b);
     }
 };
 
-template <typename T>
 struct RsProd {
     static constexpr int kMinCtas = 4;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
         const size_t n = (size_t)d.g.nx * d.g.ny * d.g.nz;
-        if constexpr (sizeof(T) == 8)
-            products_body(desc_fields<double, 6>(d.phys), desc_fields<double, 3>(d.phys), n, b, d.gx[kRsProd]);
-        else
-            products32_body(desc_fields<float, 6>(d.phys), desc_fields<float, 3>(d.phys), n, b, d.gx[kRsProd]);
+        products_body(desc_fields<double, 6>(d.phys), desc_fields<double, 3>(d.phys), n, b, d.gx[kRsProd]);
     }
 };
 
@@ -3848,7 +3842,8 @@ StageKernel ragged_kernel(int stage, bool mixed, int variant) {
     switch (stage) {
         case kRsVort:
             return mixed ? k_stage<RsVort32> : ((variant & kRvVortTc) ? k_stage<RsVort64Tc> : k_stage<RsVort64>);
-        case kRsProd: return mixed ? k_stage<RsProd<float>> : k_stage<RsProd<double>>;
+        case kRsPi: return k_stage<RsPi>;
+        case kRsProd: return k_stage<RsProd>;
         case kRsVisc:
             return mixed ? k_stage<RsVisc32> : ((variant & kRvViscTc) ? k_stage<RsVisc64Tc> : k_stage<RsVisc64>);
         case kRsPres:
@@ -3858,6 +3853,8 @@ StageKernel ragged_kernel(int stage, bool mixed, int variant) {
             return mixed ? k_stage<RsCorr32> : ((variant & kRvCorrTc) ? k_stage<RsCorr64Tc> : k_stage<RsCorr64>);
         case kRsViscMean: return k_stage<RsViscMean>;
         case kRsPresMean: return k_stage<RsPresMean>;
+        case kRsFftX: return ragged_nl_kernel(stage, mixed);
+        case kRsFftYUvw:
         case kRsFftYInv:
         case kRsFftC2R:
         case kRsFftR2C:
@@ -3865,6 +3862,8 @@ StageKernel ragged_kernel(int stage, bool mixed, int variant) {
     }
     return nullptr;
 }
+
+int ragged_threads(int stage) { return stage == kRsFftX ? nl_x_threads() : kStageThreads; }
 
 int ragged_variant(const RunDesc& d) {
     return ((d.tcmask & 1) ? kRvVortTc : 0) | ((d.tcmask & 2) ? kRvCorrTc : 0) |
@@ -3877,7 +3876,8 @@ void ragged_geometry(RunDesc& d) {
     auto cdiv = [](long long a, long long b) { return (int)((a + b - 1) / b); };
     for (int s = 0; s < kRsStages; ++s) d.gx[s] = 1;
     const int cy = fft_ct_per_cta(g.ny), rx = fft_ct_per_cta(g.nxh);
-    d.gx[kRsFftYInv] = cdiv((long long)g.nz * g.nxhp, cy);
+    d.gx[kRsFftX] = cdiv((long long)g.nz * g.ny, nl_x_rows(g.nxh));
+    d.gx[kRsFftYUvw] = d.gx[kRsFftYInv] = cdiv((long long)g.nz * g.nxhp, cy);
     d.gx[kRsFftC2R] = cdiv((long long)g.nz * g.ny, rx);
     d.gx[kRsProd] = cdiv((long long)g.nx * g.ny * g.nz, 4 * kStageThreads);
     d.gx[kRsFftR2C] = d.gx[kRsFftC2R];
@@ -3905,13 +3905,17 @@ int ragged_blocks(int stage, bool mixed, const RunDesc& d) {
     switch (stage) {
         case kRsVort:
             if (!mixed && (ragged_variant(d) & kRvVortTc))
-                return 1 + ((g.nm + kTcVortModes - 1) / kTcVortModes + d.vort_chunk - 1) / d.vort_chunk;
-            return 1 + tiles;
+                return ((g.nm + kTcVortModes - 1) / kTcVortModes + d.vort_chunk - 1) / d.vort_chunk;
+            return tiles;
+        case kRsPi: return 1;
+        case kRsFftYUvw:
         case kRsFftYInv:
-        case kRsFftC2R: return 6 * d.gx[stage];
-        case kRsFftR2C:
         case kRsFftYFwd: return 3 * d.gx[stage];
-        case kRsProd: return d.gx[stage];
+        // one x pass, or the three kernels of the FP64-pipe transforms
+        case kRsFftX: return (mixed || d.fftfx) ? d.gx[stage] : 0;
+        case kRsFftC2R: return (mixed || d.fftfx) ? 0 : 6 * d.gx[stage];
+        case kRsFftR2C: return (mixed || d.fftfx) ? 0 : 3 * d.gx[stage];
+        case kRsProd: return (mixed || d.fftfx) ? 0 : d.gx[stage];
         case kRsVisc:
             if (!mixed && (ragged_variant(d) & kRvViscTc)) return (d.ops.nq + d.gx[kRsVisc] - 1) / d.gx[kRsVisc];
             return tiles;
