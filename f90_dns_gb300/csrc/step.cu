@@ -55,6 +55,11 @@ template <typename P> __device__ __forceinline__ P* fptr(const FieldsT<P>& f, in
     return r;
 }
 
+// the same among the first three (velocity components)
+template <typename P> __device__ __forceinline__ P* fptr3(const FieldsT<P>& f, int i) {
+    return i == 0 ? f.p[0] : (i == 1 ? f.p[1] : f.p[2]);
+}
+
 // ------------------------------------------------------------------ PI / forcing
 // update_pressure_gradient_3d (3D:2488-2549) called with the namelist istart
 // (3D:1118), and calculate_bulk_velocity_3d (3D:2434-2464) from the (0,0) mode:
@@ -571,7 +576,9 @@ __device__ __forceinline__ void viscous_body(GridDev g, Ops ops, StepParams sp, 
 //      walls).
 // Two schedules (viscous_tc_pipelined).  Phased, where two CTAs share an SM:
 // per q (a) + (b) | (d) | (e) | (f) | (g), each behind a barrier, the other
-// CTA filling the waits.  Pipelined, where one CTA has the SM: while the MMAs
+// CTA filling the waits.  (One pass for (g) of q and (b) of q + 1, as below,
+// saves two barriers per q and was slower: 175 us against 152 at 128x128x65.)
+// Pipelined, where one CTA has the SM: while the MMAs
 // of q run, one pass of the CTA writes the outputs (g) of q - 1 and forms the
 // right-hand sides (b) of q + 1 (item for item in the same shared-memory
 // slots: each thread reads its results of q - 1 before it writes its
@@ -582,6 +589,10 @@ __device__ __forceinline__ void viscous_body(GridDev g, Ops ops, StepParams sp, 
 // through three, the staged inputs through two (the wall gradients and row
 // exponents, which the outputs still read, through four); the state values
 // that (g) subtracts stay in registers from (b), two sets in turn.
+// The kernel is bound by the instructions of its phases' integer chains, so a
+// thread's items of a pass and of the digits, the same for every q, are
+// divided out once, and q's wavenumbers advance without divisions: 172 -> 152 us
+// at 128x128x65 with the branch-free subtraction below.
 // (t - round(f 2^-E)) 2^E: an integer result t at the scale 2^E minus an
 // FP64 value f, exactly in integers but for the rounding of f to that scale
 // and of the final conversion; falls back to the FP64 difference where f is
@@ -589,54 +600,41 @@ __device__ __forceinline__ void viscous_body(GridDev g, Ops ops, StepParams sp, 
 // would overflow.
 __device__ __forceinline__ double tc_sub_scaled(long long t, double f, int E) {
     const long long b = __double_as_longlong(f);
-    int ex = (int)((b >> 52) & 0x7FF);
-    if (ex == 0x7FF) return i2d_scaled(t, E) - f;
-    long long m = b & 0xFFFFFFFFFFFFFLL;
-    if (ex == 0) {
-        if (m == 0) return i2d_scaled(t, E);
-        ex = 1;  // subnormal: no implicit bit
+    const int ex = (int)((b >> 52) & 0x7FF);
+    const unsigned long long m = ((unsigned long long)b & 0xFFFFFFFFFFFFFULL) | (ex ? 1ULL << 52 : 0ULL);
+    const int sh = 1075 + E - max(ex, 1);  // f 2^-E = m 2^-sh
+    // f far above the scale (f 2^-E >= 2^62) or non-finite
+    if (sh < -9 || ex == 0x7FF) return i2d_scaled(t, E) - f;
+    unsigned long long u;  // round(m 2^-sh): 2 m >> sh (zero from a shift of 64 on), or m << -sh
+    if (sh >= 0) {
+        asm("shr.u64 %0, %1, %2;" : "=l"(u) : "l"(m << 1), "r"(sh));
+        u = (u + 1) >> 1;
     } else {
-        m |= 1LL << 52;
+        u = m << -sh;
     }
-    const int sh = 1075 + E - ex;  // f 2^-E = m 2^-sh
-    long long F;
-    if (sh >= 63) F = 0;  // |f 2^-E| < 2^-10
-    else if (sh > 0) F = (m + (1LL << (sh - 1))) >> sh;
-    else if (sh >= -9) F = m << (-sh);
-    else return i2d_scaled(t, E) - f;
-    if (b < 0) F = -F;
+    const long long s = b >> 63;
+    const long long F = (long long)((u ^ (unsigned long long)s) - (unsigned long long)s);
     const long long d = (long long)((unsigned long long)t - (unsigned long long)F);
     if (((t ^ F) & (t ^ d)) < 0) return i2d_scaled(t, E) - f;  // overflow
     return i2d_scaled(d, E);
 }
 
-// Combination of one warp's TMEM lanes for 6 right-hand-side columns (H = 0:
-// columns 0 .. 5, H = 1: 6 .. 11): the 8 weight-class accumulators of each
-// column loaded back to back under one wait and combined in 64-bit integers
-// (tc_combine8), stored to sR at the lane's row as the integer T (its bits in
-// the FP64 slot; the outputs' scale 2^(e + f - 52) is applied in (g)).  The
-// two warps of a lane quadrant take one half each.
-template <int H>
-__device__ __noinline__ void tc_combine6(uint32_t lanes, double* sR, int m8, int row, bool valid) {
-    uint32_t r[kTcClasses * 6];
+// Combination of one warp's TMEM lanes for 4 right-hand-side columns from c0 (a
+// multiple of 4): the 8 weight-class accumulators of each column loaded back to
+// back under one wait and combined in 64-bit integers (tc_combine8), stored to
+// sR at the lane's row as the integer T (its bits in the FP64 slot; the outputs'
+// scale 2^(e + f - 52) is applied in (g)).
+__device__ __noinline__ void tc_combine4(uint32_t lanes, int c0, double* sR, int m8, int row, bool valid) {
+    uint32_t r[kTcClasses * 4];
 #pragma unroll
-    for (int c = 0; c < kTcClasses; ++c) {
-        const uint32_t a = lanes + (uint32_t)(c * kTcN + 6 * H);
-        if (H == 0) {
-            tc_ld4_nw(a, r + 6 * c);
-            tc_ld2_nw(a + 4, r + 6 * c + 4);
-        } else {  // each load's first column a multiple of its width
-            tc_ld2_nw(a, r + 6 * c);
-            tc_ld4_nw(a + 2, r + 6 * c + 2);
-        }
-    }
+    for (int c = 0; c < kTcClasses; ++c) tc_ld4_nw(lanes + (uint32_t)(c * kTcN + c0), r + 4 * c);
     tc_ld_wait(r);
     if (valid) {
 #pragma unroll
-        for (int j = 0; j < 6; ++j) {
-            const long long T = tc_combine8(r[j], r[6 + j], r[12 + j], r[18 + j], r[24 + j], r[30 + j], r[36 + j],
-                                            r[42 + j]);
-            sR[(6 * H + j) * m8 + row] = __longlong_as_double(T);  // the integer result, its bits
+        for (int j = 0; j < 4; ++j) {
+            const long long T = tc_combine8(r[j], r[4 + j], r[8 + j], r[12 + j], r[16 + j], r[20 + j], r[24 + j],
+                                            r[28 + j]);
+            sR[(c0 + j) * m8 + row] = __longlong_as_double(T);  // the integer result, its bits
         }
     }
 }
@@ -703,9 +701,9 @@ __host__ __device__ inline size_t viscous_tc_smem_nz(int nz) {
 
 // The schedule: phased where two CTAs share an SM (228 KB of shared memory,
 // 1 KB of it reserved per CTA), whose phases then fill each other's waits;
-// pipelined where one CTA has the SM to itself (nz >= 81).  Measured at
-// 128x128x65 (phased): 170 us phased, 174 us pipelined; at 512x384x129: 6.14
-// ms phased, 5.33 ms pipelined.
+// pipelined where one CTA has the SM to itself (nz >= 81).  Measured with 256
+// threads, at 128x128x65 (phased): 170 us phased, 174 us pipelined; at
+// 512x384x129: 6.14 ms phased, 5.33 ms pipelined.
 __host__ __device__ inline bool viscous_tc_pipelined(int nz) {
     return 2 * (viscous_tc_smem_nz<false>(nz) + 1024) > 228 * 1024;
 }
@@ -763,6 +761,21 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     const int ncore = t.ncore_e + t.ncore_o;
     const bool staged = viscous_tc_staged<kPipe>(t, nz);
     const int nitems = 6 * he;  // (b) and (g): (mode, component, level pair)
+    // item i = threadIdx.x + p blockDim.x, p = 0, 1, as mode | component | level
+    // pair: the same for every q, so divided out once
+    struct Item {
+        int mi, comp, k;
+    };
+    auto decode = [&](int i) {
+        const int mi = i >= 3 * he ? 1 : 0, r = i - mi * 3 * he;
+        const int comp = r >= 2 * he ? 2 : (r >= he ? 1 : 0);
+        return (r - comp * he) | comp << 8 | mi << 10;
+    };
+    const int it0 = decode(threadIdx.x), it1 = decode(threadIdx.x + blockDim.x);
+    auto item = [&](int i, int p) {
+        const int d = p == 0 ? it0 : (p == 1 ? it1 : decode(i));
+        return Item{d >> 10, (d >> 8) & 3, d & 255};
+    };
     struct QInfo {
         int kya, kx, nmode;
     };
@@ -773,21 +786,28 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
         r.nmode = (r.kya > 0 && 2 * r.kya != g.ny) ? 2 : 1;
         return r;
     };
+    auto qnext = [&](QInfo r) {  // qinfo of the next operator index, without its division
+        if (++r.kx == g.nxhp) {
+            r.kx = 0;
+            ++r.kya;
+            r.nmode = (r.kya > 0 && 2 * r.kya != g.ny) ? 2 : 1;
+        }
+        return r;
+    };
     // cp.async of the inputs of operator index q (both modes' columns of u, v,
     // w and of the sources; a missing second mode is not read): one warp per
     // column, its lanes over the levels; one commit group per q, empty past
     // the CTA's last q or when the inputs are not staged
-    auto stage = [&](int q) {
+    auto stage = [&](int q, const QInfo& qi) {
         if (staged && q < q1) {
             const int rel = q - q0;
-            const QInfo qi = qinfo(q);
             double2* sP = pslot(rel);
             const int lane = threadIdx.x & 31;
             for (int r = threadIdx.x >> 5; r < 2 * qi.nmode * 3; r += blockDim.x >> 5) {
                 const int comp = r % 3, r2 = r / 3;
                 const int mi = r2 % qi.nmode, fld = r2 / qi.nmode;
                 const int m = (mi ? g.ny - qi.kya : qi.kya) * g.nxhp + qi.kx;
-                const double2* src = (fld ? fptr(Src, comp) : fptr(F, comp)) + m;
+                const double2* src = (fld ? fptr3(Src, comp) : fptr3(F, comp)) + m;
                 double2* dst = sP + (size_t)((fld * 2 + mi) * 3 + comp) * nz;
                 for (int z = lane; z < nz; z += 32) cp_async16(dst + z, src + (size_t)z * g.nm);
             }
@@ -827,14 +847,13 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     // (b) item i of q: the folded right-hand sides of column pair 6 mi + 2 comp
     // + (0 re, 1 im) at level pair k into the q's buffer; returns the state
     // values at the two levels (kept for (g)) and the keys of the values
-    auto rhs_item = [&](int q, const QInfo& qi, int i, double2& v1o, double2& v2o, unsigned& kre, unsigned& kim) {
+    auto rhs_item = [&](int q, const QInfo& qi, const Item& it, double2& v1o, double2& v2o, unsigned& kre,
+                        unsigned& kim) {
         const int rel = q - q0;
         const double2* sP = pslot(rel);
         const double2* sGP = sGP4 + 8 * gslot(rel);
         double* sR = rslot(rel);
-        const int mi = i / (3 * he);
-        const int r = i - mi * 3 * he;
-        const int comp = r / he, k = r - comp * he;
+        const int mi = it.mi, comp = it.comp, k = it.k;
         double2 fe = make_double2(0.0, 0.0), fo = fe;
         if (mi < qi.nmode) {
             const int ky = mi ? g.ny - qi.kya : qi.kya;
@@ -842,8 +861,8 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             // the F and source columns of this mode: staged, or read from
             // global memory one level (a plane) apart
             const size_t st = staged ? 1 : (size_t)g.nm;
-            const double2* fc = staged ? sP + (size_t)(mi * 3 + comp) * nz : fptr(F, comp) + m;
-            const double2* sc = staged ? sP + (size_t)((2 + mi) * 3 + comp) * nz : fptr(Src, comp) + m;
+            const double2* fc = staged ? sP + (size_t)(mi * 3 + comp) * nz : fptr3(F, comp) + m;
+            const double2* sc = staged ? sP + (size_t)((2 + mi) * 3 + comp) * nz : fptr3(Src, comp) + m;
             const double2 f1 = fc[0], fn = fc[(size_t)(nz - 1) * st];
             const double2 v1 = fc[(size_t)k * st], v2 = k < ho ? fc[(size_t)(nz - 1 - k) * st] : v1;
             v1o = v1;
@@ -883,19 +902,17 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     // E = e_k + f_c - 52 and F = round(f 2^-E), exactly in integers but for
     // that one rounding of f and the final conversion; v1, v2: the state
     // values at levels k, nz-1-k (read again from F past the kept items)
-    auto out_item = [&](int q, const QInfo& qi, int i, int p, double2 v1, double2 v2) {
+    auto out_item = [&](int q, const QInfo& qi, const Item& it, int p, double2 v1, double2 v2) {
         const int rel = q - q0;
         const double2* sGP = sGP4 + 8 * gslot(rel);
         const int* sEq = sEq4 + gslot(rel) * m8;
         const double* sR = rslot(rel);
         const unsigned* sK = kslot(rel);
-        const int mi = i / (3 * he);
-        const int r = i - mi * 3 * he;
-        const int comp = r / he, k = r - comp * he;
+        const int mi = it.mi, comp = it.comp, k = it.k;
         const int ky = mi ? g.ny - qi.kya : qi.kya;
         const int m = ky * g.nxhp + qi.kx;
         const int c0 = 6 * mi + 2 * comp;
-        double2* oc = fptr(Out, comp);
+        double2* oc = fptr3(Out, comp);
         const size_t o1 = (size_t)k * g.nm + m, o2 = (size_t)(nz - 1 - k) * g.nm + m;
         if (k == 0) {
             double2 bc1 = make_double2(0.0, 0.0), bc2 = bc1;
@@ -910,7 +927,7 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             return;
         }
         if (p >= 2) {
-            const double2* fc = fptr(F, comp);
+            const double2* fc = fptr3(F, comp);
             v1 = fc[o1];
             v2 = k < ho ? fc[o2] : v1;
         }
@@ -943,8 +960,7 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     // right-hand sides (b) of qb (if qb < q1), item for item, then the column
     // keys of qb: per warp and column a warp maximum and one shared atomic;
     // the pipelined schedule then swaps kA and kB
-    auto pass = [&](int qg, int qb) {
-        const QInfo ig = qinfo(max(qg, q0)), ib = qinfo(min(qb, q1 - 1));
+    auto pass = [&](int qg, const QInfo& ig, int qb, const QInfo& ib) {
         const bool dog = qg >= q0, dob = qb < q1;
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
         for (int p = 0; p * (int)blockDim.x < nitems; ++p) {
@@ -959,9 +975,10 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
                     v1 = kA1[1];
                     v2 = kA2[1];
                 }
-                if (dog && i < ig.nmode * 3 * he) out_item(qg, ig, i, p, v1, v2);
+                const Item it = item(i, p);
+                if (dog && it.mi < ig.nmode) out_item(qg, ig, it, p, v1, v2);
                 if (dob) {
-                    rhs_item(qb, ib, i, v1, v2, kre, kim);
+                    rhs_item(qb, ib, it, v1, v2, kre, kim);
                     if (p == 0) {
                         kA1[0] = v1;
                         kA2[0] = v2;
@@ -973,10 +990,13 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             }
             const int ifirst = w * 32 + p * (int)blockDim.x;
             if (dob && ifirst < nitems) {  // uniform over the warp
-                const int glast = min(ifirst + 31, nitems - 1) / he;
-                const int mygrp = i < nitems ? i / he : -1;
+                // column pair 2 g, 2 g + 1 of item (mode, component): g = 3 mode + component
+                const Item it = item(i, p);
+                const int mygrp = i < nitems ? 3 * it.mi + it.comp : -1;
+                const int gfirst = __shfl_sync(0xffffffffu, mygrp, 0);
+                const int glast = __reduce_max_sync(0xffffffffu, mygrp);
                 unsigned* sK = kslot(qb - q0);
-                for (int gi = ifirst / he; gi <= glast; ++gi) {  // column pair 2 gi, 2 gi + 1
+                for (int gi = gfirst; gi <= glast; ++gi) {
                     const unsigned re = __reduce_max_sync(0xffffffffu, mygrp == gi ? kre : 0u);
                     const unsigned im = __reduce_max_sync(0xffffffffu, mygrp == gi ? kim : 0u);
                     if (lane == 0) {
@@ -1003,19 +1023,32 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     // 8-row group for 8 columns, so its 4-byte stores fall in distinct
     // shared-memory banks but for columns 8 apart (the bank of (n, k) in a
     // core matrix is 4 (n mod 8) + (k mod 8)/2)
+    struct Dig {
+        int col, r0, r1, off;  // column, rows of the two values (-1: padding), offset of the digit pair
+    };
+    auto dig = [&](int i) {
+        const int kp = i & 3, cc = i >> 2;
+        Dig d;
+        d.col = cc % 12;
+        const int kk = (cc / 12) * 8 + 2 * kp;
+        d.r0 = i < 12 * (t.kt / 2) ? tc_k_row(t, kk) : -1;
+        d.r1 = tc_k_row(t, kk + 1);
+        d.off = tc_core_off(d.col, kk, t.kt);
+        return d;
+    };
+    const Dig dg0 = dig(threadIdx.x), dg1 = dig(threadIdx.x + blockDim.x);
     auto digits = [&](int q) {
         const int rel = q - q0;
         const double* sR = rslot(rel);
         const unsigned* sK = kslot(rel);
-        for (int i = threadIdx.x; i < 12 * (t.kt / 2); i += blockDim.x) {
-            const int kp = i & 3, cc = i >> 2;
-            const int c = cc % 12, kk = (cc / 12) * 8 + 2 * kp;
-            const int r0 = tc_k_row(t, kk), r1 = tc_k_row(t, kk + 1);
-            if (r0 < 0) continue;  // padding K rows: zeroed once at the start, never written
-            const int f = tc_exponent_key(sK[c]);
+        for (int p = 0; p * (int)blockDim.x < 12 * (t.kt / 2); ++p) {
+            const Dig d = p == 0 ? dg0 : (p == 1 ? dg1 : dig(threadIdx.x + p * blockDim.x));
+            if (d.r0 < 0) continue;  // padding K rows: zeroed once at the start, never written
+            const int f = tc_exponent_key(sK[d.col]);
+            const double* col = sR + d.col * m8;
             __half2 h[kTcSlices];
-            tc_digit_pairs(tc_fixed(sR[c * m8 + r0], f), r1 < 0 ? 0 : tc_fixed(sR[c * m8 + r1], f), h);
-            __half2* dst = reinterpret_cast<__half2*>(sB + tc_core_off(c, kk, t.kt));
+            tc_digit_pairs(tc_fixed(col[d.r0], f), d.r1 < 0 ? 0 : tc_fixed(col[d.r1], f), h);
+            __half2* dst = reinterpret_cast<__half2*>(sB + d.off);
 #pragma unroll
             for (int s = 0; s < kTcSlices; ++s) dst[s * (b_halves / 2)] = h[s];
         }
@@ -1060,33 +1093,21 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     };
     // (f) combine the accumulators of each row of q into its result buffer:
     // warp w reads TMEM lane quadrant w % 4 (lanes 32 (w % 4) .. +31); block
-    // E's rows are lanes 0 .. e8, block O's lanes 64 .. 64 + o8.  A quadrant
-    // holding rows of one block splits its 12 columns between its two warps
-    // (6 each); one holding rows of both blocks (nz = 129: lanes 64 .. 71 of
-    // E) gives each warp one block.
+    // E's rows are lanes 0 .. e8, block O's lanes 64 .. 64 + o8 (a quadrant
+    // holds rows of both at nz = 129: lanes 64 .. 71 of E).  The warps of a
+    // quadrant take its (block, 4-column group) items.
     auto combine = [&](int q) {
         double* sR = rslot(q - q0);
-        const int w = threadIdx.x >> 5;
-        if (w < 8) {
-            const int quad = w & 3, half = w >> 2;
-            const bool hasE = 32 * quad < t.e8;
-            const bool hasO = quad >= 2 && 32 * quad < 64 + t.o8;
-            const int lane = 32 * quad + (threadIdx.x & 31);
-            const uint32_t lanes = tmem + ((uint32_t)(32 * quad) << 16);
-            if (hasE || hasO) {
-                const int blk = (hasE && hasO) ? half : (hasO ? 1 : 0);
-                const bool valid = blk ? (lane >= 64 && lane - 64 < t.o8) : lane < t.e8;
-                const int row = blk ? t.e8 + (lane - 64) : lane;
-                const uint32_t lb = lanes + (uint32_t)(blk * kTcDCols);
-                if (hasE && hasO) {
-                    tc_combine6<0>(lb, sR, m8, row, valid);
-                    tc_combine6<1>(lb, sR, m8, row, valid);
-                } else if (half == 0) {
-                    tc_combine6<0>(lb, sR, m8, row, valid);
-                } else {
-                    tc_combine6<1>(lb, sR, m8, row, valid);
-                }
-            }
+        const int w = threadIdx.x >> 5, quad = w & 3;
+        const bool hasE = 32 * quad < t.e8;
+        const bool hasO = quad >= 2 && 32 * quad < 64 + t.o8;
+        const int lane = 32 * quad + (threadIdx.x & 31);
+        const uint32_t lanes = tmem + ((uint32_t)(32 * quad) << 16);
+        const int nit = ((int)hasE + (int)hasO) * 3, nw = ((int)(blockDim.x >> 5) - quad + 3) >> 2;
+        for (int it = w >> 2; it < nit; it += nw) {
+            const int blk = (hasE && it < 3) ? 0 : 1, c0 = (it % 3) * 4;
+            const bool valid = blk ? (lane >= 64 && lane - 64 < t.o8) : lane < t.e8;
+            tc_combine4(lanes + (uint32_t)(blk * kTcDCols), c0, sR, m8, blk ? t.e8 + (lane - 64) : lane, valid);
         }
     };
     bool ok = true;
@@ -1103,19 +1124,28 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             if (next) tc_mbar_wait(&mbar[1], par ^ 1u, 1 << 22);
         }
     };
+    // the MMAs of q done (polled by one warp that issues none of them: the others
+    // wait at the barrier and leave their issue slots to the other CTA) and both
+    // copies landed
+    auto mmas_done = [&](uint32_t par) {
+        const bool w = (int)(threadIdx.x >> 5) != (kPipe ? 0 : 2) || tc_mbar_wait(&mbar[0], par, mlimit);
+        return __syncthreads_and(w) && landed[0] && landed[1];
+    };
+    QInfo qc = qinfo(min(q0, ops.nq - 1));  // of q
     if (!kPipe) {
         // phased: per q, (a) + (b) | (d) | (e) | (f) | (g), the staged inputs
         // of q + 1 arriving during (d)-(g)
-        if (q0 < q1) stage(q0);
+        if (q0 < q1) stage(q0, qc);
         for (int q = q0; q < q1; ++q) {
             const int rel = q - q0;
             const uint32_t par = (uint32_t)(rel & 1);
+            const QInfo qn = qnext(qc);
             cp_async_wait_all();
-            __syncthreads();  // this q's staged inputs, from every thread's copies
-            copy_op(q);
-            pass(q0 - 1, q);
             __syncthreads();
-            if (q + 1 < q1) stage(q + 1);  // the staging buffer is free again
+            copy_op(q);
+            pass(q0 - 1, qc, q, qc);
+            __syncthreads();
+            stage(q + 1, qn);  // the staging buffer is free again
             if (threadIdx.x < kTcN) kslot(rel + 1)[threadIdx.x] = 0u;  // (g) of q - 1 read them last
             digits(q);
             tc_fence_proxy();
@@ -1123,7 +1153,7 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             __syncthreads();
             tc_fence_after();
             issue(par);
-            const bool done = __syncthreads_and(tc_mbar_wait(&mbar[0], par, mlimit)) && landed[0] && landed[1];
+            const bool done = mmas_done(par);
             tc_fence_after();
             if (!done) {
                 timed_out(par, false);
@@ -1132,20 +1162,22 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             }
             combine(q);
             tc_fence_before();
-            __syncthreads();
-            pass(q, q1);
-            __syncthreads();  // shared buffers are reused by the next q
+            __syncthreads();  // results of q; TMEM free for the MMAs of q + 1
+            tc_fence_after();
+            pass(q, qc, q1, qn);
+            qc = qn;
         }
     } else if (q0 < q1) {
         // pipelined
-        stage(q0);
-        stage(q0 + 1);
+        QInfo qn = qnext(qc), qp = qc;  // of q + 1, q - 1
+        stage(q0, qc);
+        stage(q0 + 1, qn);
         cp_async_wait_one();  // q0's inputs
         __syncthreads();
         copy_op(q0);
-        pass(q0 - 1, q0);
+        pass(q0 - 1, qp, q0, qc);
         __syncthreads();  // q0's right-hand sides and column keys; its staging buffer is free
-        stage(q0 + 2);
+        stage(q0 + 2, qnext(qn));
         digits(q0);
         cp_async_wait_one();  // q0 + 1's inputs
         tc_fence_proxy();
@@ -1169,15 +1201,15 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
                     }
                 }
             }
-            pass(q - 1, q + 1);  // beside the MMAs of q
-            const bool done = __syncthreads_and(tc_mbar_wait(&mbar[0], par, mlimit)) && landed[0] && landed[1];
+            pass(q - 1, qp, q + 1, qn);  // beside the MMAs of q
+            const bool done = mmas_done(par);
             tc_fence_after();
             if (!done) {
                 timed_out(par, *nextc != 0);
                 ok = false;
                 break;  // uniform: no TMEM read, no further MMA
             }
-            stage(q + 3);  // into the buffers (b) of q + 1 and (g) of q - 1 read last
+            stage(q + 3, qnext(qnext(qn)));  // into the buffers (b) of q + 1 and (g) of q - 1 read last
             combine(q);
             if (threadIdx.x < kTcN) kslot(q + 2 - q0)[threadIdx.x] = 0u;  // (g) of q - 1 read them last
             if (q + 1 < q1) digits(q + 1);
@@ -1186,8 +1218,11 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
             tc_fence_before();
             __syncthreads();  // results of q, digits of q + 1; TMEM free for the MMAs of q + 1
             tc_fence_after();
+            qp = qc;
+            qc = qn;
+            qn = qnext(qn);
         }
-        if (ok) pass(q1 - 1, q1);  // the outputs of the last q
+        if (ok) pass(q1 - 1, qp, q1, qc);  // the outputs of the last q
     }
     cp_async_wait_all();  // a stage issued before a timeout lands before the CTA leaves
     tc_fence_before();
@@ -1196,8 +1231,14 @@ __device__ __forceinline__ void viscous_tc_body(const GridDev& g, const Ops& ops
     if (threadIdx.x < 32) tc_dealloc(tmem, 2 * kTcDCols);
 }
 
+// Threads per CTA: 256 where two CTAs share an SM; 512 where one has it to
+// itself, so that the CUDA-core phases, which take most of an operator index's
+// time, have 16 warps either way (512x384x129: 5.45 ms with 256 threads, 4.47 ms with 512, 3.92
+// ms with the index work below; 96x192x81: 388, 291 and 280 us).
+constexpr int vtc_threads(bool pipe) { return pipe ? 512 : 256; }
+
 template <bool kPipe>
-__global__ void __launch_bounds__(256, 2) k_viscous_tc(GridDev g, Ops ops, StepParams sp, Fields F, Fields Src,
+__global__ void __launch_bounds__(vtc_threads(kPipe), kPipe ? 1 : 2) k_viscous_tc(GridDev g, Ops ops, StepParams sp, Fields F, Fields Src,
                                                        const double2* __restrict__ GP,
                                                        const dns3d_pi_state* __restrict__ pi, Fields Out, int qpb,
                                                        int* err) {
@@ -1569,8 +1610,13 @@ struct CorrTcOp {
     }
 };
 
-template <class Op>
-__global__ void __launch_bounds__(kTcVortThreads, 2) k_dz_tc(GridDev g, Ops ops, Op op, int chunk, int* err) {
+// kThreads: 512 where two CTAs share an SM, 1024 where the D1 image leaves room
+// for one (nz >= 81) and the operator has one field, whose outputs bound the
+// tile (projection at 512x384x129: 1.28 ms with 512 threads, 1.14 ms with 1024;
+// at 96x192x81 90 and 86 us).  The vorticity's two fields leave 1024 threads
+// two tiles' worth of levels short of work: 1.82 and 1.83 ms, 130 and 131 us.
+template <class Op, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_dz_tc(GridDev g, Ops ops, Op op, int chunk, int* err) {
     constexpr int kModes = kTcVortCols / (2 * Op::kFields);
     const int ntiles = (g.nm + kModes - 1) / kModes;
     const int t0 = blockIdx.x * chunk;
@@ -3315,9 +3361,11 @@ cudaError_t prepare_step_kernels(const GridDev& g) {
     if ((e = set_smem(k_divergence, (size_t)g.nz * tile_cols(g, 1) * sizeof(double2)))) return e;
     if ((e = set_smem(k_viscous_tc<false>, 0))) return e;
     if ((e = set_smem(k_viscous_tc<true>, 0))) return e;
-    if ((e = set_smem(k_dz_tc<VortTcOp>, 0))) return e;
-    if ((e = set_smem(k_dz_tc<CorrTcOp>, 0))) return e;
-    if ((e = set_smem(k_dz_tc<PresRhsTcOp>, 0))) return e;
+    if ((e = set_smem(k_dz_tc<VortTcOp, kTcVortThreads>, 0))) return e;
+    if ((e = set_smem(k_dz_tc<CorrTcOp, kTcVortThreads>, 0))) return e;
+    if ((e = set_smem(k_dz_tc<CorrTcOp, 2 * kTcVortThreads>, 0))) return e;
+    if ((e = set_smem(k_dz_tc<PresRhsTcOp, kTcVortThreads>, 0))) return e;
+    if ((e = set_smem(k_dz_tc<PresRhsTcOp, 2 * kTcVortThreads>, 0))) return e;
     if ((e = set_smem(k_pressure_solve, 0))) return e;
     if ((e = set_smem(k_pcg_poisson, pcg_smem(g)))) return e;
     if ((e = set_smem(k_pcg_helmholtz, pcg_smem(g)))) return e;
@@ -3438,12 +3486,15 @@ int tc_q_per_cta(int nq) { return std::max(1, (nq + 2 * 152 - 1) / (2 * 152)); }
 cudaError_t launch_viscous_tc(const GridDev& g, const Ops& ops, const StepParams& sp, Fields F, Fields Src,
                               const double2* GP, const dns3d_pi_state* pi, Fields Out, int* err, cudaStream_t s) {
     if (!ops.tcA || !ops.tcE || !viscous_tc_fits(g)) return cudaErrorInvalidValue;
-    const int qpb = tc_q_per_cta(ops.nq);
+    const bool pipe = viscous_tc_pipelined(g.nz);
+    // one wave of the CTAs that are resident at once
+    const int qpb = pipe ? std::max(1, (ops.nq + 151) / 152) : tc_q_per_cta(ops.nq);
     const int nb = (ops.nq + qpb - 1) / qpb;
-    if (viscous_tc_pipelined(g.nz))
-        k_viscous_tc<true><<<nb, 256, viscous_tc_smem(g), s>>>(g, ops, sp, F, Src, GP, pi, Out, qpb, err);
+    if (pipe)
+        k_viscous_tc<true><<<nb, vtc_threads(true), viscous_tc_smem(g), s>>>(g, ops, sp, F, Src, GP, pi, Out, qpb, err);
     else
-        k_viscous_tc<false><<<nb, 256, viscous_tc_smem(g), s>>>(g, ops, sp, F, Src, GP, pi, Out, qpb, err);
+        k_viscous_tc<false><<<nb, vtc_threads(false), viscous_tc_smem(g), s>>>(g, ops, sp, F, Src, GP, pi, Out, qpb,
+                                                                                err);
     return cudaGetLastError();
 }
 
@@ -3453,9 +3504,9 @@ size_t vorticity_tc_smem(const GridDev& g) {
 }
 
 bool vorticity_tc_fits(const GridDev& g) {
-    return tc_supported(g.nz) && vorticity_tc_smem(g) <= smem_limit(k_dz_tc<VortTcOp>) &&
-           vorticity_tc_smem(g) <= smem_limit(k_dz_tc<CorrTcOp>) &&
-           vorticity_tc_smem(g) <= smem_limit(k_dz_tc<PresRhsTcOp>);
+    return tc_supported(g.nz) && vorticity_tc_smem(g) <= smem_limit(k_dz_tc<VortTcOp, kTcVortThreads>) &&
+           vorticity_tc_smem(g) <= smem_limit(k_dz_tc<CorrTcOp, kTcVortThreads>) &&
+           vorticity_tc_smem(g) <= smem_limit(k_dz_tc<PresRhsTcOp, kTcVortThreads>);
 }
 
 // Tiles (of `modes` modes) per CTA: at least 4 (the D1 image is copied once
@@ -3472,7 +3523,12 @@ cudaError_t launch_dz_tc(const GridDev& g, const Ops& ops, const Op& op, int* er
     constexpr int kModes = kTcVortCols / (2 * Op::kFields);
     const int ntiles = (g.nm + kModes - 1) / kModes;
     const int chunk = tc_dz_chunk(g.nm, kModes);
-    k_dz_tc<Op><<<(ntiles + chunk - 1) / chunk, kTcVortThreads, vorticity_tc_smem(g), s>>>(g, ops, op, chunk, err);
+    const size_t sm = vorticity_tc_smem(g);
+    constexpr int kWide = Op::kFields == 1 ? 2 * kTcVortThreads : kTcVortThreads;
+    if (2 * (sm + 1024) > 228 * 1024)
+        k_dz_tc<Op, kWide><<<(ntiles + chunk - 1) / chunk, kWide, sm, s>>>(g, ops, op, chunk, err);
+    else
+        k_dz_tc<Op, kTcVortThreads><<<(ntiles + chunk - 1) / chunk, kTcVortThreads, sm, s>>>(g, ops, op, chunk, err);
     return cudaGetLastError();
 }
 
