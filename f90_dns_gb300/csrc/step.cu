@@ -60,6 +60,15 @@ template <typename P> __device__ __forceinline__ P* fptr3(const FieldsT<P>& f, i
     return i == 0 ? f.p[0] : (i == 1 ? f.p[1] : f.p[2]);
 }
 
+// t / tc and t - tc (t / tc) for a tile width: a shift where tc is a power of
+// two (every width the autotuner tries), in place of the integer division's
+// two dozen instructions per item.
+struct TileDiv {
+    int tc, sh;
+};
+__device__ __forceinline__ TileDiv tile_div(int tc) { return {tc, (tc & (tc - 1)) ? -1 : 31 - __clz(tc)}; }
+__device__ __forceinline__ int tile_row(TileDiv d, int t) { return d.sh >= 0 ? t >> d.sh : t / d.tc; }
+
 // ------------------------------------------------------------------ PI / forcing
 // update_pressure_gradient_3d (3D:2488-2549) called with the namelist istart
 // (3D:1118), and calculate_bulk_velocity_3d (3D:2434-2464) from the (0,0) mode:
@@ -2330,8 +2339,9 @@ __global__ void __launch_bounds__(256) k_divergence(GridDev g, Ops ops, const do
 // feed the FP32 inverse transforms of the nonlinear term.
 __device__ __forceinline__ void fold_load32(float2* tile, const double2* __restrict__ src, const GridDev& g,
                                             int m0, int tc, int he, int ho) {
+    const TileDiv td = tile_div(tc);
     for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
+        const int k = tile_row(td, t), c = t - k * tc;
         const int m = m0 + c;
         float2 fe = make_float2(0.f, 0.f), fo = fe;
         if (m < g.nm) {
@@ -2377,11 +2387,12 @@ __device__ __forceinline__ void vorticity_mixed_body(GridDev g, MixedOps mx, Ops
     const int nz = g.nz, he = ops.he, ho = ops.ho;
     float2* tv = tu + nz * tc;
     const int m0 = bx * tc;
+    const TileDiv td = tile_div(tc);
     fold_load32(tu, U, g, m0, tc, he, ho);
     fold_load32(tv, V, g, m0, tc, he, ho);
     __syncthreads();
     for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
+        const int k = tile_row(td, t), c = t - k * tc;
         const int m = m0 + c;
         if (m >= g.nm) continue;
         float2 due, dve, duo = make_float2(0.f, 0.f), dvo = duo;
@@ -2412,7 +2423,7 @@ __device__ __forceinline__ void vorticity_mixed_body(GridDev g, MixedOps mx, Ops
     }
 }
 
-__global__ void __launch_bounds__(256) k_vorticity_mixed(GridDev g, MixedOps mx, Ops ops,
+__global__ void __launch_bounds__(512) k_vorticity_mixed(GridDev g, MixedOps mx, Ops ops,
                                                          const double2* __restrict__ U,
                                                          const double2* __restrict__ V,
                                                          const double2* __restrict__ W, FFields out, int tc) {
@@ -2467,6 +2478,7 @@ __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops o
     float4* tw = reinterpret_cast<float4*>(ty + tsz);   // [tc] wall terms
     float* tk = reinterpret_cast<float*>(tw + tc);      // [tc] k^2 (-1: skip; <= -2: masked source)
     const int m0 = bx * tc;
+    const TileDiv td = tile_div(tc);
     if (stage_mats) {  // the eigenbasis matrices (a persistent CTA stages them once)
         const float4* A = reinterpret_cast<const float4*>(mx.AeT);
         for (int t = threadIdx.x; t < hei * (pe4 / 4); t += blockDim.x) sAe[t] = __ldg(&A[t]);
@@ -2481,7 +2493,7 @@ __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops o
     for (int comp = 0; comp < 3; ++comp) {
         // fold the interior column: even rows k < hei, odd rows pe4 + k
         for (int t = threadIdx.x; t < pe4 * tc; t += blockDim.x) {
-            const int k = t / tc, c = t - k * tc;
+            const int k = tile_row(td, t), c = t - k * tc;
             const int m = m0 + c;
             float2 se = make_float2(0.f, 0.f), de = se, ss = se, ds = se;
             if (m < g.nm && k < hei) {
@@ -2540,7 +2552,7 @@ __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops o
         __syncthreads();
         // ut, st for 4 eigen-rows of one block (even or odd)
         for (int t = threadIdx.x; t < (nr / 4) * tc; t += blockDim.x) {
-            const int jb = t / tc, c = t - jb * tc;
+            const int jb = tile_row(td, t), c = t - jb * tc;
             const int j0 = 4 * jb;
             float k2 = tk[c];
             if (k2 == -1.f) {
@@ -2591,7 +2603,7 @@ __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops o
         __syncthreads();
         // back to the interior levels: 4 output pairs per item
         for (int t = threadIdx.x; t < (pe4 / 4) * tc; t += blockDim.x) {
-            const int ib = t / tc, c = t - ib * tc;
+            const int ib = tile_row(td, t), c = t - ib * tc;
             const int m = m0 + c;
             if (tk[c] == -1.f) continue;
             const int i0 = 4 * ib;
@@ -2695,8 +2707,9 @@ __device__ __forceinline__ double df_value(DF s) { return f2d(s.hi) + f2d(s.lo);
 // (skip0: mode 0 is left zero and not read, e.g. while another kernel writes it)
 __device__ __forceinline__ void fold_load_df(float4* tile, const double2* __restrict__ src, const GridDev& g,
                                              int m0, int tc, int he, int ho, bool skip0 = false) {
+    const TileDiv td = tile_div(tc);
     for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
+        const int k = tile_row(td, t), c = t - k * tc;
         const int m = m0 + c;
         double2 fe = make_double2(0.0, 0.0), fo = fe;
         if (m < g.nm && !(skip0 && m == 0)) {
@@ -2716,6 +2729,49 @@ __device__ __forceinline__ void fold_load_df(float4* tile, const double2* __rest
             tile[(he + k) * tc + c] = make_float4(ox.hi, ox.lo, oy.hi, oy.lo);
         }
     }
+}
+
+// df_split with integer operations alone (an FP64 subtraction takes the time
+// of 80 FP32 ones here): the mantissa's top 24 bits, rounded half up, and the
+// signed rest.  Non-finite x gives NaN.
+__device__ __forceinline__ DF df_split_bits(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7FFu), fe = e - 896;  // biased float exponent
+    const unsigned sg = hi & 0x80000000u;
+    const unsigned rest = lo & 0x1FFFFFFFu, up = rest >> 28;
+    const unsigned m = (((hi & 0xFFFFFu) << 3) | (lo >> 29)) + up;  // without the implicit bit
+    const float r = (float)((int)rest - (int)(up << 29));  // x = (2^23 + m) 2^(e-1046) + r 2^(e-1075)
+    DF d;
+    d.hi = fe > 0 ? __uint_as_float(sg | (((unsigned)fe << 23) + m)) : __uint_as_float(sg);
+    const unsigned rb = __float_as_uint(r);
+    const int le = (int)((rb >> 23) & 0xFFu) + e - 1075;  // biased exponent of the rest
+    d.lo = (rb != 0u && le > 0) ? __uint_as_float((rb + ((unsigned)(e - 1075) << 23)) ^ sg) : 0.f;
+    if (e >= 896 + 255) d.hi = d.lo = __uint_as_float(0x7FC00000u);
+    return d;
+}
+__device__ __forceinline__ DF df_neg(DF a) { return {-a.hi, -a.lo}; }
+// a + b (Knuth's two-sum of the high parts)
+__device__ __forceinline__ DF df_add(DF a, DF b) {
+    const float t = __fadd_rn(a.hi, b.hi), z = __fsub_rn(t, a.hi);
+    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(t, z)), __fsub_rn(b.hi, z));
+    return {t, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
+}
+__device__ __forceinline__ void df_mac(DF& s, DF a, DF b) { df_mac(s, a.hi, a.lo, b.hi, b.lo); }
+
+// Dot products of double-floats with a bound known beforehand: the high sum
+// starts at c = 3 2^q with 2^q >= sum |a_i b_i|, so it stays in [2^(q+1), 2^(q+2)]
+// and is always the larger addend: t = fma(a, b, s) and t - s are then exact but
+// for t's rounding, which fma(a, b, s - t) recovers -- 6 FP32 instructions per
+// term against the 12 of df_mac.  Errors are 2^-46 of the bound: for D1.w* of
+// evolved channel fields at most 1.2e-11 (nz = 33) to 3.5e-10 (nz = 193) of the
+// column's largest right-hand side, whose rounding to FP32 after it is 6e-8.
+__device__ __forceinline__ void df_dot(DF& s, float ahi, float alo, float bhi, float blo) {
+    const float t = fmaf(ahi, bhi, s.hi);
+    const float z = __fsub_rn(s.hi, t);
+    s.lo = __fadd_rn(s.lo, fmaf(ahi, bhi, z));
+    s.lo = fmaf(ahi, blo, s.lo);
+    s.lo = fmaf(alo, bhi, s.lo);
+    s.hi = t;
 }
 
 // anti_apply_df's even and odd parts before their sum and difference:
@@ -2788,14 +2844,16 @@ __device__ __forceinline__ Pair sym_apply_df(const float2* __restrict__ Ae, cons
 }
 
 // phi~_j = -(V'^T b)_j / (l'_j + k^2) of the folded right-hand sides tb of a
-// mode tile, 4 eigen-rows of one block per thread, into tp.
+// mode tile, 4 eigen-rows of one block per thread, into tp; sk2 [tc]: k^2 of the
+// tile's modes.
 __device__ __forceinline__ void pressure_mixed_forward(const GridDev& g, const MixedOps& mx, const Ops& ops,
                                                        const float* PAe, const float* PAo, const float2* tb,
-                                                       float2* tp, int m0, int tc) {
+                                                       float2* tp, const float* sk2, int m0, int tc) {
+    const TileDiv td = tile_div(tc);
     const int he = ops.he, ho = ops.ho;
     const int pe4 = mx.phe4, po4 = mx.pho4, nbe = pe4 / 4, nbo = po4 / 4;
     for (int t = threadIdx.x; t < (nbe + nbo) * tc; t += blockDim.x) {
-        const int jb = t / tc, c = t - jb * tc;
+        const int jb = tile_row(td, t), c = t - jb * tc;
         const int m = m0 + c;
         const bool even = jb < nbe;
         const int j0 = even ? 4 * jb : 4 * (jb - nbe);
@@ -2806,6 +2864,7 @@ __device__ __forceinline__ void pressure_mixed_forward(const GridDev& g, const M
             const int len = even ? he : ho, ld4 = even ? nbe : nbo;
             const float4* __restrict__ A = reinterpret_cast<const float4*>(even ? PAe : PAo) + j0 / 4;
             const float2* b = tb + (even ? 0 : pe4 * tc) + c;
+#pragma unroll 4
             for (int i = 0; i < len; ++i) {
                 const float4 e = __ldg(&A[(size_t)i * ld4]);
                 const float2 v = b[i * tc];
@@ -2814,8 +2873,7 @@ __device__ __forceinline__ void pressure_mixed_forward(const GridDev& g, const M
                 acc[2].x = fmaf(e.z, v.x, acc[2].x); acc[2].y = fmaf(e.z, v.y, acc[2].y);
                 acc[3].x = fmaf(e.w, v.x, acc[3].x); acc[3].y = fmaf(e.w, v.y, acc[3].y);
             }
-            const int ky = m / g.nxhp, kx = m - ky * g.nxhp;
-            const float k2 = d2f(__ldg(&ops.ksq[mode_q(ky, kx, g.ny, g.nxhp)]));
+            const float k2 = sk2[c];
             const float* lam = even ? mx.plame : mx.plamo;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -2830,66 +2888,44 @@ __device__ __forceinline__ void pressure_mixed_forward(const GridDev& g, const M
     }
 }
 
-// phi = pe + po, dphi/dz = dze + dzo at levels (i, nz-1-i) from tp, 4 rows i
-// per thread: pe = PBe phi~e, po = PBo phi~o, dze = PDe phi~o, dzo = PDo
-// phi~e; stored into PHI, PHIZ, or added to them (a correction).
+// phi = pe + po, dphi/dz = dze + dzo at levels (i, nz-1-i) from tp, 4 rows i of
+// one of the two per thread: pe = PBe phi~e, po = PBo phi~o, dze = PDe phi~o,
+// dzo = PDo phi~e; stored into PHI, PHIZ, or added to them (a correction).
 template <bool kAdd>
 __device__ __forceinline__ void pressure_mixed_back(const GridDev& g, const MixedOps& mx, const Ops& ops,
                                                     const float2* tp, double2* __restrict__ PHI,
                                                     double2* __restrict__ PHIZ, int m0, int tc) {
     const int nz = g.nz, he = ops.he, ho = ops.ho;
     const int pe4 = mx.phe4, po4 = mx.pho4, nbe = pe4 / 4, nbo = po4 / 4;
-    for (int t = threadIdx.x; t < nbe * tc; t += blockDim.x) {
-        const int ib = t / tc, c = t - ib * tc;
+    const TileDiv td = tile_div(tc);
+    for (int t = threadIdx.x; t < 2 * nbe * tc; t += blockDim.x) {
+        const int row = tile_row(td, t), c = t - row * tc;
         const int m = m0 + c;
         if (m >= g.nm || m == 0) continue;
+        const bool dz = row >= nbe;
+        const int ib = dz ? row - nbe : row;
         const int i0 = 4 * ib;
-        float2 pe[4], po[4], de[4], dd[4];
+        float2 ev[4], od[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) { pe[q] = make_float2(0.f, 0.f); po[q] = pe[q]; de[q] = pe[q]; dd[q] = pe[q]; }
+        for (int q = 0; q < 4; ++q) { ev[q] = make_float2(0.f, 0.f); od[q] = ev[q]; }
+        auto rows = [&](const float* M, int nb, const float2* q, int len, float2* acc) {
+            const float4* __restrict__ B = reinterpret_cast<const float4*>(M) + ib;
+#pragma unroll 4
+            for (int j = 0; j < len; ++j) {
+                const float4 a = __ldg(&B[(size_t)j * nb]);
+                const float2 v = q[j * tc];
+                acc[0].x = fmaf(a.x, v.x, acc[0].x); acc[0].y = fmaf(a.x, v.y, acc[0].y);
+                acc[1].x = fmaf(a.y, v.x, acc[1].x); acc[1].y = fmaf(a.y, v.y, acc[1].y);
+                acc[2].x = fmaf(a.z, v.x, acc[2].x); acc[2].y = fmaf(a.z, v.y, acc[2].y);
+                acc[3].x = fmaf(a.w, v.x, acc[3].x); acc[3].y = fmaf(a.w, v.y, acc[3].y);
+            }
+        };
         const float2* qe = tp + c;
-        const float2* qo = tp + pe4 * tc + c;
-        {
-            const float4* __restrict__ B = reinterpret_cast<const float4*>(mx.PBe) + ib;
-            for (int j = 0; j < he; ++j) {
-                const float4 a = __ldg(&B[(size_t)j * nbe]);
-                const float2 v = qe[j * tc];
-                pe[0].x = fmaf(a.x, v.x, pe[0].x); pe[0].y = fmaf(a.x, v.y, pe[0].y);
-                pe[1].x = fmaf(a.y, v.x, pe[1].x); pe[1].y = fmaf(a.y, v.y, pe[1].y);
-                pe[2].x = fmaf(a.z, v.x, pe[2].x); pe[2].y = fmaf(a.z, v.y, pe[2].y);
-                pe[3].x = fmaf(a.w, v.x, pe[3].x); pe[3].y = fmaf(a.w, v.y, pe[3].y);
-            }
-            const float4* __restrict__ D = reinterpret_cast<const float4*>(mx.PDe) + ib;
-            for (int j = 0; j < ho; ++j) {
-                const float4 a = __ldg(&D[(size_t)j * nbe]);
-                const float2 v = qo[j * tc];
-                de[0].x = fmaf(a.x, v.x, de[0].x); de[0].y = fmaf(a.x, v.y, de[0].y);
-                de[1].x = fmaf(a.y, v.x, de[1].x); de[1].y = fmaf(a.y, v.y, de[1].y);
-                de[2].x = fmaf(a.z, v.x, de[2].x); de[2].y = fmaf(a.z, v.y, de[2].y);
-                de[3].x = fmaf(a.w, v.x, de[3].x); de[3].y = fmaf(a.w, v.y, de[3].y);
-            }
-        }
-        if (ib < nbo) {
-            const float4* __restrict__ B = reinterpret_cast<const float4*>(mx.PBo) + ib;
-            for (int j = 0; j < ho; ++j) {
-                const float4 a = __ldg(&B[(size_t)j * nbo]);
-                const float2 v = qo[j * tc];
-                po[0].x = fmaf(a.x, v.x, po[0].x); po[0].y = fmaf(a.x, v.y, po[0].y);
-                po[1].x = fmaf(a.y, v.x, po[1].x); po[1].y = fmaf(a.y, v.y, po[1].y);
-                po[2].x = fmaf(a.z, v.x, po[2].x); po[2].y = fmaf(a.z, v.y, po[2].y);
-                po[3].x = fmaf(a.w, v.x, po[3].x); po[3].y = fmaf(a.w, v.y, po[3].y);
-            }
-            const float4* __restrict__ D = reinterpret_cast<const float4*>(mx.PDo) + ib;
-            for (int j = 0; j < he; ++j) {
-                const float4 a = __ldg(&D[(size_t)j * nbo]);
-                const float2 v = qe[j * tc];
-                dd[0].x = fmaf(a.x, v.x, dd[0].x); dd[0].y = fmaf(a.x, v.y, dd[0].y);
-                dd[1].x = fmaf(a.y, v.x, dd[1].x); dd[1].y = fmaf(a.y, v.y, dd[1].y);
-                dd[2].x = fmaf(a.z, v.x, dd[2].x); dd[2].y = fmaf(a.z, v.y, dd[2].y);
-                dd[3].x = fmaf(a.w, v.x, dd[3].x); dd[3].y = fmaf(a.w, v.y, dd[3].y);
-            }
-        }
-        auto put = [&](size_t o, double2* F, float x, float y) {
+        const float2* qo = qe + pe4 * tc;
+        rows(dz ? mx.PDe : mx.PBe, nbe, dz ? qo : qe, dz ? ho : he, ev);
+        if (ib < nbo) rows(dz ? mx.PDo : mx.PBo, nbo, dz ? qe : qo, dz ? he : ho, od);
+        double2* __restrict__ F = dz ? PHIZ : PHI;
+        auto put = [&](size_t o, float x, float y) {
             const double2 v = make_double2(f2d(x), f2d(y));
             if (kAdd) {
                 const double2 o0 = F[o];
@@ -2904,14 +2940,10 @@ __device__ __forceinline__ void pressure_mixed_back(const GridDev& g, const Mixe
             if (i >= he) break;
             const size_t o1 = (size_t)i * g.nm + m;
             if (i < ho) {
-                const size_t o2 = (size_t)(nz - 1 - i) * g.nm + m;
-                put(o1, PHI, pe[q].x + po[q].x, pe[q].y + po[q].y);
-                put(o2, PHI, pe[q].x - po[q].x, pe[q].y - po[q].y);
-                put(o1, PHIZ, de[q].x + dd[q].x, de[q].y + dd[q].y);
-                put(o2, PHIZ, de[q].x - dd[q].x, de[q].y - dd[q].y);
+                put(o1, ev[q].x + od[q].x, ev[q].y + od[q].y);
+                put((size_t)(nz - 1 - i) * g.nm + m, ev[q].x - od[q].x, ev[q].y - od[q].y);
             } else {
-                put(o1, PHI, pe[q].x, pe[q].y);
-                put(o1, PHIZ, de[q].x, de[q].y);
+                put(o1, ev[q].x, ev[q].y);
             }
         }
     }
@@ -2933,6 +2965,14 @@ __device__ __forceinline__ void pressure_mixed_back(const GridDev& g, const Mixe
 // stored phi with S applied in double-float (about 2^-48 relative, against
 // the 2^-24 of the FP32 solve), and the FP32 solve of P d = r is added to
 // phi and dphi/dz: the Galerkin residual drops from ~1e-7 to ~1e-13 of b.
+// Bytes of pressure_mixed_body's shared memory before the refinement's FP64
+// right-hand side.
+__host__ __device__ inline size_t pressure_mixed_base(int nz, int tc) {
+    const int ho = nz / 2, he = nz - ho, rows = (he + 3) / 4 * 4 + (ho + 3) / 4 * 4;
+    return ((size_t)(nz + 1) * tc * sizeof(float4) + 2 * (size_t)rows * tc * sizeof(float2) + 2 * (size_t)tc * sizeof(float) +
+            15) / 16 * 16;
+}
+
 template <bool kRefine>
 __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops ops, StepParams sp,
                                                     const double2* __restrict__ US,
@@ -2944,48 +2984,141 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
     const int nz = g.nz, he = ops.he, ho = ops.ho;
     const int pe4 = mx.phe4, po4 = mx.pho4;
     float4* tw = reinterpret_cast<float4*>(smraw);              // folded w* (double-float)  [nz][tc]
-    float2* tb = reinterpret_cast<float2*>(tw + nz * tc);       // folded rhs: s [pe4][tc], d [po4][tc]
+    float4* ta = tw + nz * tc;                                  // (i ax / 2, i ay / 2) as double-floats [tc]
+    float2* tb = reinterpret_cast<float2*>(ta + tc);            // folded rhs: s [pe4][tc], d [po4][tc]
     float2* tp = tb + (pe4 + po4) * tc;                         // phi~: even [pe4][tc], odd [po4][tc]
-    double2* bt = reinterpret_cast<double2*>(tp + (pe4 + po4) * tc);  // FP64 rhs [nz][tc] (refinement)
+    float* tk = reinterpret_cast<float*>(tp + (pe4 + po4) * tc);  // k^2 [tc]
+    unsigned* tm = reinterpret_cast<unsigned*>(tk + tc);        // largest q |re|, q |im| of the folded column (float bits)
+    double2* bt = reinterpret_cast<double2*>(smraw + pressure_mixed_base(nz, tc));  // FP64 rhs [nz][tc] (refinement)
     const int m0 = bx * tc;
-    fold_load_df(tw, WS, g, m0, tc, he, ho);
+    const bool strong = !kRefine && !sp.weak_form;
+    const TileDiv td = tile_div(tc);
+    for (int c = threadIdx.x; c < tc; c += blockDim.x) {
+        const int m = min(m0 + c, g.nm - 1);
+        const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
+        const DF ax = df_split_bits(0.5 * mi.ax), ay = df_split_bits(0.5 * mi.ay);
+        ta[c] = make_float4(ax.hi, ax.lo, ay.hi, ay.lo);
+        tk[c] = d2f(__ldg(&ops.ksq[mode_q(mi.ky, mi.kx, g.ny, g.nxhp)]));
+        tm[c] = 0u;
+    }
     for (int t = threadIdx.x; t < (pe4 - he) * tc; t += blockDim.x) tb[he * tc + t] = make_float2(0.f, 0.f);
     for (int t = threadIdx.x; t < (po4 - ho) * tc; t += blockDim.x) tb[(pe4 + ho) * tc + t] = make_float2(0.f, 0.f);
-    __syncthreads();
-    const float2* __restrict__ Ae = sp.weak_form ? mx.W1e_df : mx.D1e_df;
-    const float2* __restrict__ Ao = sp.weak_form ? mx.W1o_df : mx.D1o_df;
-    // right-hand side pair (k, nz-1-k), folded in FP64 before the rounding
-    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
-        const int m = m0 + c;
-        float2 fs = make_float2(0.f, 0.f), fd = fs;
-        double2 b1 = make_double2(0.0, 0.0), b2 = b1;
-        if (m < g.nm && m != 0) {
-            const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
-            if (!kRefine && !sp.weak_form) {
-                // the folded strong-form right-hand side divided by 2 w_k / dt
-                // (the scaled forward operators PAeS, PAoS carry that factor):
-                // (b_k +- b_k') dt / (2 w_k) = i (ax/2)(u_k +- u_k') +
-                // i (ay/2)(v_k +- v_k') + (ye | yo), the mid level
-                // i (ax/2) u_k + i (ay/2) v_k + ye / 2; ye, yo the even and
-                // odd parts of D1.w* -- 20 FP64 operations per level pair
-                // instead of 36
-                const double4 y = anti_apply_df_parts(Ae, Ao, tw, k, c, tc, he, ho);
-                const double hax = 0.5 * mi.ax, hay = 0.5 * mi.ay;
-                const size_t o1 = (size_t)k * g.nm + m;
-                const double2 u1 = US[o1], v1 = VS[o1];
+    if (strong) {
+        __syncthreads();  // tm zeroed
+        // w* as double-floats, folded, and each column's largest component
+        // weighted by q (MixedOps)
+        for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
+            const int k = tile_row(td, t), c = t - k * tc;
+            const int m = m0 + c;
+            float4 fe = make_float4(0.f, 0.f, 0.f, 0.f), fo = fe;
+            if (m < g.nm) {
+                const double2 a = WS[(size_t)k * g.nm + m];
+                const DF ax = df_split_bits(a.x), ay = df_split_bits(a.y);
+                fe = make_float4(ax.hi, ax.lo, ay.hi, ay.lo);
                 if (k < ho) {
-                    const size_t o2 = (size_t)(nz - 1 - k) * g.nm + m;
-                    const double2 u2 = US[o2], v2 = VS[o2];
-                    const double2 up = make_double2(u1.x + u2.x, u1.y + u2.y), um = make_double2(u1.x - u2.x, u1.y - u2.y);
-                    const double2 vp = make_double2(v1.x + v2.x, v1.y + v2.y), vm = make_double2(v1.x - v2.x, v1.y - v2.y);
-                    fs = make_float2(d2f(fma(-hax, up.y, fma(-hay, vp.y, y.x))), d2f(fma(hax, up.x, fma(hay, vp.x, y.y))));
-                    fd = make_float2(d2f(fma(-hax, um.y, fma(-hay, vm.y, y.z))), d2f(fma(hax, um.x, fma(hay, vm.x, y.w))));
-                } else {
-                    fs = make_float2(d2f(fma(-hax, u1.y, fma(-hay, v1.y, 0.5 * y.x))),
-                                     d2f(fma(hax, u1.x, fma(hay, v1.x, 0.5 * y.y))));
+                    const double2 b = WS[(size_t)(nz - 1 - k) * g.nm + m];
+                    const DF bx_ = df_split_bits(b.x), by = df_split_bits(b.y);
+                    const DF px = df_add(ax, bx_), py = df_add(ay, by);
+                    const DF mx_ = df_add(ax, df_neg(bx_)), my = df_add(ay, df_neg(by));
+                    fe = make_float4(px.hi, px.lo, py.hi, py.lo);
+                    fo = make_float4(mx_.hi, mx_.lo, my.hi, my.lo);
                 }
-            } else {
+            }
+            tw[t] = fe;
+            if (k < ho) tw[(he + k) * tc + c] = fo;
+            const unsigned mag = 0x7FFFFFFFu;
+            const unsigned big = max(max(__float_as_uint(fe.x) & mag, __float_as_uint(fe.z) & mag),
+                                     max(__float_as_uint(fo.x) & mag, __float_as_uint(fo.z) & mag));
+            atomicMax(&tm[c], __float_as_uint(__uint_as_float(big) * __ldg(&mx.D1q[k])));
+        }
+        __syncthreads();
+        // The folded strong-form right-hand side divided by 2 w_k / dt (the
+        // scaled forward operators PAeS, PAoS carry that factor), all in
+        // double-float: (b_k +- b_k') dt / (2 w_k) = i (ax/2)(u_k +- u_k') +
+        // i (ay/2)(v_k +- v_k') + (ye | yo), the mid level i (ax/2) u_k +
+        // i (ay/2) v_k + ye / 2; ye, yo the even and odd parts of D1.w*.
+        // With the combination in FP64 (20 operations per level pair, each the
+        // time of 80 FP32 ones) the kernel took 63 us at 128x128x65, 354 us at
+        // 256x256x97; now 48 and 307.
+        for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
+            const int k = tile_row(td, t), c = t - k * tc;
+            const int m = m0 + c;
+            float2 fs = make_float2(0.f, 0.f), fd = fs;
+            if (m < g.nm && m != 0) {
+                const size_t o1 = (size_t)k * g.nm + m, o2 = (size_t)(nz - 1 - k) * g.nm + m;
+                const double2 u1 = US[o1], v1 = VS[o1], u2 = US[o2], v2 = VS[o2];
+                // the column's largest weighted component as a power of two above it
+                const float cm = __uint_as_float((tm[c] & 0x7F800000u) + 0x00800000u);
+                const float ce = 3.f * cm * __ldg(&mx.D1eC[k]);
+                DF yex{ce, 0.f}, yey{ce, 0.f}, yox{0.f, 0.f}, yoy{0.f, 0.f};
+                {
+                    const float2* er = mx.D1e_df + (size_t)k * ho;
+                    const float4* f = tw + he * tc + c;
+#pragma unroll 4
+                    for (int j = 0; j < ho; ++j) {
+                        const float2 a = __ldg(&er[j]);
+                        const float4 b = f[j * tc];
+                        df_dot(yex, a.x, a.y, b.x, b.y);
+                        df_dot(yey, a.x, a.y, b.z, b.w);
+                    }
+                    yex.hi -= ce;
+                    yey.hi -= ce;
+                }
+                const float4 ma = ta[c];
+                const DF hax{ma.x, ma.y}, hay{ma.z, ma.w}, nax = df_neg(hax), nay = df_neg(hay);
+                const DF u1x = df_split_bits(u1.x), u1y = df_split_bits(u1.y);
+                const DF v1x = df_split_bits(v1.x), v1y = df_split_bits(v1.y);
+                if (k < ho) {
+                    const float co = 3.f * cm * __ldg(&mx.D1oC[k]);
+                    yox.hi = yoy.hi = co;
+                    const float2* orow = mx.D1o_df + (size_t)k * he;
+                    const float4* f = tw + c;
+#pragma unroll 4
+                    for (int j = 0; j < he; ++j) {
+                        const float2 a = __ldg(&orow[j]);
+                        const float4 b = f[j * tc];
+                        df_dot(yox, a.x, a.y, b.x, b.y);
+                        df_dot(yoy, a.x, a.y, b.z, b.w);
+                    }
+                    yox.hi -= co;
+                    yoy.hi -= co;
+                    const DF u2x = df_split_bits(u2.x), u2y = df_split_bits(u2.y);
+                    const DF v2x = df_split_bits(v2.x), v2y = df_split_bits(v2.y);
+                    df_mac(yex, nax, df_add(u1y, u2y));
+                    df_mac(yex, nay, df_add(v1y, v2y));
+                    df_mac(yey, hax, df_add(u1x, u2x));
+                    df_mac(yey, hay, df_add(v1x, v2x));
+                    df_mac(yox, nax, df_add(u1y, df_neg(u2y)));
+                    df_mac(yox, nay, df_add(v1y, df_neg(v2y)));
+                    df_mac(yoy, hax, df_add(u1x, df_neg(u2x)));
+                    df_mac(yoy, hay, df_add(v1x, df_neg(v2x)));
+                    fd = make_float2(yox.hi + yox.lo, yoy.hi + yoy.lo);
+                } else {
+                    yex = DF{0.5f * yex.hi, 0.5f * yex.lo};
+                    yey = DF{0.5f * yey.hi, 0.5f * yey.lo};
+                    df_mac(yex, nax, u1y);
+                    df_mac(yex, nay, v1y);
+                    df_mac(yey, hax, u1x);
+                    df_mac(yey, hay, v1x);
+                }
+                fs = make_float2(yex.hi + yex.lo, yey.hi + yey.lo);
+            }
+            tb[k * tc + c] = fs;
+            if (k < ho) tb[(pe4 + k) * tc + c] = fd;
+        }
+    } else {
+        fold_load_df(tw, WS, g, m0, tc, he, ho);
+        __syncthreads();
+        const float2* __restrict__ Ae = sp.weak_form ? mx.W1e_df : mx.D1e_df;
+        const float2* __restrict__ Ao = sp.weak_form ? mx.W1o_df : mx.D1o_df;
+        // right-hand side pair (k, nz-1-k), folded in FP64 before the rounding
+        for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
+            const int k = tile_row(td, t), c = t - k * tc;
+            const int m = m0 + c;
+            float2 fs = make_float2(0.f, 0.f), fd = fs;
+            double2 b1 = make_double2(0.0, 0.0), b2 = b1;
+            if (m < g.nm && m != 0) {
+                const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
                 const Pair dz = anti_apply_df(Ae, Ao, tw, k, c, tc, he, ho);
                 b1 = pressure_rhs(g, ops, sp, k, m, mi, US, VS, dz.a);
                 if (k < ho) {
@@ -2996,17 +3129,16 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
                     fs = make_float2(d2f(b1.x), d2f(b1.y));
                 }
             }
-        }
-        tb[k * tc + c] = fs;
-        if (k < ho) tb[(pe4 + k) * tc + c] = fd;
-        if (kRefine) {
-            bt[k * tc + c] = b1;
-            if (k < ho) bt[(nz - 1 - k) * tc + c] = b2;
+            tb[k * tc + c] = fs;
+            if (k < ho) tb[(pe4 + k) * tc + c] = fd;
+            if (kRefine) {
+                bt[k * tc + c] = b1;
+                if (k < ho) bt[(nz - 1 - k) * tc + c] = b2;
+            }
         }
     }
     __syncthreads();
-    const bool scaled = !kRefine && !sp.weak_form;
-    pressure_mixed_forward(g, mx, ops, scaled ? mx.PAeS : mx.PAe, scaled ? mx.PAoS : mx.PAo, tb, tp, m0, tc);
+    pressure_mixed_forward(g, mx, ops, strong ? mx.PAeS : mx.PAe, strong ? mx.PAoS : mx.PAo, tb, tp, tk, m0, tc);
     __syncthreads();
     pressure_mixed_back<false>(g, mx, ops, tp, PHI, PHIZ, m0, tc);
     if (!kRefine) return;
@@ -3015,7 +3147,7 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
     fold_load_df(tw, PHI, g, m0, tc, he, ho, true);
     __syncthreads();
     for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
+        const int k = tile_row(td, t), c = t - k * tc;
         const int m = m0 + c;
         float2 fs = make_float2(0.f, 0.f), fd = fs;
         if (m < g.nm && m != 0) {
@@ -3039,13 +3171,13 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
         if (k < ho) tb[(pe4 + k) * tc + c] = fd;
     }
     __syncthreads();
-    pressure_mixed_forward(g, mx, ops, mx.PAe, mx.PAo, tb, tp, m0, tc);
+    pressure_mixed_forward(g, mx, ops, mx.PAe, mx.PAo, tb, tp, tk, m0, tc);
     __syncthreads();
     pressure_mixed_back<true>(g, mx, ops, tp, PHI, PHIZ, m0, tc);
 }
 
 template <bool kRefine>
-__global__ void __launch_bounds__(256) k_pressure_mixed(GridDev g, MixedOps mx, Ops ops, StepParams sp,
+__global__ void __launch_bounds__(512) k_pressure_mixed(GridDev g, MixedOps mx, Ops ops, StepParams sp,
                                                         const double2* __restrict__ US,
                                                         const double2* __restrict__ VS,
                                                         const double2* __restrict__ WS,
@@ -3282,9 +3414,16 @@ int tile_cols_mixed(const GridDev& g) {
 }
 
 size_t pressure_mixed_smem(const GridDev& g, int tc) {
-    const int ho = g.nz / 2, he = g.nz - ho;
-    return (size_t)g.nz * tc * sizeof(float4) + 2 * (size_t)(pad4(he) + pad4(ho)) * tc * sizeof(float2) +
+    return pressure_mixed_base(g.nz, tc) +
            (g.refine ? (size_t)g.nz * tc * sizeof(double2) : 0);  // the FP64 right-hand side kept for the refinement
+}
+
+// Threads of k_vorticity_mixed: as few equal rounds of at most 512 threads as
+// cover its items (256 threads leave a last round of 16 items where an odd
+// he x tc is 2 x 256 + 16, as at nz = 65).  256x256x97: 136 -> 123 us.
+int tile_threads(int items) {
+    const int rounds = std::max(1, (items + 511) / 512);
+    return std::max(64, ((items + rounds - 1) / rounds + 31) / 32 * 32);
 }
 
 namespace {
@@ -3561,7 +3700,7 @@ cudaError_t launch_vorticity_mixed(const GridDev& g, const MixedOps& mx, const O
                                    const double2* V, const double2* W, FFields out, cudaStream_t s) {
     const int tc = tile_width(g, kTileVortM);
     const size_t sm = 2 * (size_t)g.nz * tc * sizeof(float2);
-    k_vorticity_mixed<<<(g.nm + tc - 1) / tc, 256, sm, s>>>(g, mx, ops, U, V, W, out, tc);
+    k_vorticity_mixed<<<(g.nm + tc - 1) / tc, tile_threads((g.nz - g.nz / 2) * tc), sm, s>>>(g, mx, ops, U, V, W, out, tc);
     return cudaGetLastError();
 }
 
@@ -3579,10 +3718,14 @@ cudaError_t launch_pressure_mixed(const GridDev& g, const MixedOps& mx, const Op
                                   double2* PHIZ, cudaStream_t s) {
     const int tc = tile_width(g, kTilePresM);
     const size_t sm = pressure_mixed_smem(g, tc);
+    // 16 warps hide the latency of the matrix rows (us, 256 -> 512 threads:
+    // 128x128x65 51.4 -> 48.3, 192x96x58 refined 110.8 -> 110.6, 256x256x97
+    // 324 -> 307, 64x48x40 18.4 either way)
+    const int nt = 512;
     if (sp.refine)
-        k_pressure_mixed<true><<<(g.nm + tc - 1) / tc, 256, sm, s>>>(g, mx, ops, sp, US, VS, WS, PHI, PHIZ, tc);
+        k_pressure_mixed<true><<<(g.nm + tc - 1) / tc, nt, sm, s>>>(g, mx, ops, sp, US, VS, WS, PHI, PHIZ, tc);
     else
-        k_pressure_mixed<false><<<(g.nm + tc - 1) / tc, 256, sm, s>>>(g, mx, ops, sp, US, VS, WS, PHI, PHIZ, tc);
+        k_pressure_mixed<false><<<(g.nm + tc - 1) / tc, nt, sm, s>>>(g, mx, ops, sp, US, VS, WS, PHI, PHIZ, tc);
     return cudaGetLastError();
 }
 
