@@ -153,10 +153,11 @@ __device__ __forceinline__ void fold_load(double2* tile, const double2* __restri
 
 // ye = sum_j E[k][j] * in[j] over j < len (E row-major with leading dim len);
 // in is a folded tile part with column stride tc.
+template <int kUnroll = 4>
 __device__ __forceinline__ double2 fold_dot(const double* __restrict__ erow, const double2* in, int len, int tc,
                                             int c) {
     double2 acc = make_double2(0.0, 0.0);
-#pragma unroll 4
+#pragma unroll kUnroll
     for (int j = 0; j < len; ++j) {
         const double e = __ldg(&erow[j]);
         const double2 a = in[j * tc + c];
@@ -185,6 +186,51 @@ __device__ __forceinline__ Pair anti_apply(const double* __restrict__ De, const 
     }
     return p;
 }
+// kLanes lanes per output pair.  1: one lane has both levels.  2, side by side:
+// the lane of parity 0 sums the even part and gets the level z = k, the lane of
+// parity 1 the odd part and the level nz-1-k, in the order of one lane's sums:
+// the same bits, half as long chains of loads and FP64 operations and twice the
+// warps, for 3% more FP64 time (he = ho + 1 where nz is odd) and the exchange.
+// All lanes of a warp run an item loop's iterations together.
+template <int kLanes>
+struct PairItem {
+    int par, idx;  // parity, pair index
+    __device__ __forceinline__ explicit PairItem(int t) : par(kLanes == 2 ? t & 1 : 0), idx(kLanes == 2 ? t >> 1 : t) {}
+    // f(level, which) for the lane's levels: z = k (which 0) and z = nz-1-k (1)
+    template <typename Fn>
+    __device__ __forceinline__ void levels(int k, int ho, int nz, const Fn& f) const {
+        if (kLanes == 2) {
+            f(par ? nz - 1 - k : k, par);
+        } else {
+            f(k, 0);
+            if (k < ho) f(nz - 1 - k, 1);
+        }
+    }
+    __device__ __forceinline__ bool has(int k, int he, int ho) const { return k < (par ? ho : he); }
+};
+// e + o and e - o of the two lanes' own values: the sum in lane 0, the
+// difference in lane 1
+__device__ __forceinline__ double2 pair_level(double2 own, int par) {
+    const double2 o = make_double2(__shfl_xor_sync(0xffffffffu, own.x, 1), __shfl_xor_sync(0xffffffffu, own.y, 1));
+    return par ? make_double2(o.x - own.x, o.y - own.y) : make_double2(own.x + o.x, own.y + o.y);
+}
+template <int kLanes>
+__device__ __forceinline__ Pair anti_levels(const double* __restrict__ De, const double* __restrict__ Do,
+                                            const double2* tile, int k, int c, int par, bool live, int tc, int he,
+                                            int ho) {
+    Pair y;
+    y.a = y.b = make_double2(0.0, 0.0);
+    if (kLanes == 1) {
+        if (live) y = anti_apply(De, Do, tile, k, c, tc, he, ho);
+        return y;
+    }
+    // one loop for both parities: selected operands, not diverging branches
+    const int len = par ? he : ho;
+    if (live) y.a = fold_dot<8>((par ? Do : De) + (size_t)k * len, tile + (par ? 0 : he * tc), len, tc, c);
+    y.a = y.b = pair_level(y.a, par);
+    return y;
+}
+
 __device__ __forceinline__ Pair sym_apply(const double* __restrict__ Ae, const double* __restrict__ Ao,
                                           const double2* tile, int k, int c, int tc, int he, int ho) {
     const double2 ye = fold_dot(Ae + (size_t)k * he, tile, he, tc, c);
@@ -204,6 +250,7 @@ __device__ __forceinline__ double2 c2sub(double2 a, double2 b) { return make_dou
 
 // ------------------------------------------------------------------ vorticity
 // omega = (wy - vz, uz - wx, vx - uy)  (3D:1077-1079), spectrally.
+template <int kLanes>
 __device__ __forceinline__ void vorticity_body(GridDev g, Ops ops, const double2* __restrict__ U,
                                                const double2* __restrict__ V,
                                                const double2* __restrict__ W,
@@ -217,16 +264,16 @@ __device__ __forceinline__ void vorticity_body(GridDev g, Ops ops, const double2
     fold_load(tu, U, g, m0, tc, he, ho);
     fold_load(tv, V, g, m0, tc, he, ho);
     __syncthreads();
-    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
+    for (int t0 = 0; t0 < kLanes * he * tc; t0 += blockDim.x) {
+        const PairItem<kLanes> it(t0 + threadIdx.x);
+        const int k = it.idx / tc, c = it.idx - k * tc;
         const int m = m0 + c;
-        if (m >= g.nm) continue;
-        const Pair du = anti_apply(ops.D1e, ops.D1o, tu, k, c, tc, he, ho);
-        const Pair dv = anti_apply(ops.D1e, ops.D1o, tv, k, c, tc, he, ho);
+        const bool live = it.has(k, he, ho) && m < g.nm;
+        const Pair du = anti_levels<kLanes>(ops.D1e, ops.D1o, tu, k, c, it.par, live, tc, he, ho);
+        const Pair dv = anti_levels<kLanes>(ops.D1e, ops.D1o, tv, k, c, it.par, live, tc, he, ho);
+        if (!live) continue;
         const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
-        const int npt = (k < ho) ? 2 : 1;
-        for (int p = 0; p < npt; ++p) {
-            const int z = p ? nz - 1 - k : k;
+        it.levels(k, ho, nz, [&](int z, int p) {
             const size_t o = (size_t)z * g.nm + m;
             const double2 w = W[o], u = U[o], v = V[o];
             const double2 wy = i_times(mi.ay, w), wx = i_times(mi.ax, w);
@@ -234,16 +281,17 @@ __device__ __forceinline__ void vorticity_body(GridDev g, Ops ops, const double2
             OX[o] = c2sub(wy, p ? dv.b : dv.a);
             OY[o] = c2sub(p ? du.b : du.a, wx);
             OZ[o] = c2sub(vx, uy);
-        }
+        });
     }
 }
 
+template <int kLanes>
 __global__ void __launch_bounds__(256) k_vorticity(GridDev g, Ops ops, const double2* __restrict__ U,
                                                    const double2* __restrict__ V,
                                                    const double2* __restrict__ W,
                                                    double2* __restrict__ OX, double2* __restrict__ OY,
                                                    double2* __restrict__ OZ, int tc) {
-    vorticity_body(g, ops, U, V, W, OX, OY, OZ, tc, blockIdx.x);
+    vorticity_body<kLanes>(g, ops, U, V, W, OX, OY, OZ, tc, blockIdx.x);
 }
 
 // ------------------------------------------------------------------ products
@@ -263,30 +311,30 @@ __global__ void k_products(RFields in, RFields out, size_t n) {
     products_body(in, out, n, blockIdx.x, gridDim.x);
 }
 
+// sum_j A[j len] b[j ld]: one row of a transposed square operator of `len` rows
+template <int kUnroll = 4>
+__device__ __forceinline__ double2 inv_dot(const double* __restrict__ A, const double2* b, int len, int ld) {
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll kUnroll
+    for (int j = 0; j < len; ++j) {
+        const double a = __ldg(&A[(size_t)j * len]);
+        const double2 v = b[j * ld];
+        acc.x = fma(a, v.x, acc.x);
+        acc.y = fma(a, v.y, acc.y);
+    }
+    return acc;
+}
+
 // Per-mode folded inverse x = G b for the output pair k of column c:
 // GT points at [GeT (he x he) | GoT (ho x ho)] stored transposed
 // (GeT[j][k] = Ge[k][j]) so that threads of consecutive k read consecutive
 // addresses.  bt is the folded rhs tile.
 __device__ __forceinline__ Pair inv_apply(const double* __restrict__ GT, const double2* bt, int k, int c, int tc,
                                           int he, int ho) {
-    double2 xe = make_double2(0.0, 0.0), xo = xe;
-#pragma unroll 4
-    for (int j = 0; j < he; ++j) {
-        const double gv = __ldg(&GT[(size_t)j * he + k]);
-        const double2 b = bt[j * tc + c];
-        xe.x = fma(gv, b.x, xe.x);
-        xe.y = fma(gv, b.y, xe.y);
-    }
+    const double2 xe = inv_dot(GT + k, bt + c, he, tc);
     Pair p;
     if (k < ho) {
-        const double* __restrict__ GoT = GT + (size_t)he * he;
-#pragma unroll 4
-        for (int j = 0; j < ho; ++j) {
-            const double gv = __ldg(&GoT[(size_t)j * ho + k]);
-            const double2 b = bt[(he + j) * tc + c];
-            xo.x = fma(gv, b.x, xo.x);
-            xo.y = fma(gv, b.y, xo.y);
-        }
+        const double2 xo = inv_dot(GT + (size_t)he * he + k, bt + he * tc + c, ho, tc);
         p.a = make_double2(xe.x + xo.x, xe.y + xo.y);
         p.b = make_double2(xe.x - xo.x, xe.y - xo.y);
     } else {
@@ -1732,6 +1780,7 @@ __global__ void __launch_bounds__(256) k_poisson_residual(GridDev g, Ops ops, St
     }
 }
 
+template <int kLanes>
 __device__ __forceinline__ void pressure_body(GridDev g, Ops ops, StepParams sp,
                                               const double2* __restrict__ US,
                                               const double2* __restrict__ VS,
@@ -1748,7 +1797,7 @@ __device__ __forceinline__ void pressure_body(GridDev g, Ops ops, StepParams sp,
     __syncthreads();
     const double* __restrict__ Ae = sp.weak_form ? ops.W1e : ops.D1e;
     const double* __restrict__ Ao = sp.weak_form ? ops.W1o : ops.D1o;
-    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
+    for (int t = threadIdx.x; kLanes == 1 && t < he * tc; t += blockDim.x) {
         const int k = t / tc, c = t - k * tc;
         const int m = m0 + c;
         if (m >= g.nm) {
@@ -1771,23 +1820,25 @@ __device__ __forceinline__ void pressure_body(GridDev g, Ops ops, StepParams sp,
         }
         if (sp.rhs_only && m != 0) PHI[(size_t)k * g.nm + m] = b1;
     }
+    for (int t0 = 0; kLanes == 2 && t0 < 2 * he * tc; t0 += blockDim.x) {
+        const PairItem<2> it(t0 + threadIdx.x);
+        const int k = it.idx / tc, c = it.idx - k * tc;
+        const int m = m0 + c, z = it.par ? nz - 1 - k : k;
+        const bool row = it.has(k, he, ho), live = row && m < g.nm;
+        double2 b = anti_levels<2>(Ae, Ao, tw, k, c, it.par, live, tc, he, ho).a;
+        if (live) {
+            b = pressure_rhs(g, ops, sp, z, m, mode_info(g, m, ops.xw, ops.yw), US, VS, b);
+            if (m == 0) bpin[z] = b;
+            if (sp.rhs_only && m != 0) PHI[(size_t)z * g.nm + m] = b;
+        } else {
+            b = make_double2(0.0, 0.0);
+        }
+        b = pair_level(b, it.par);  // b_k + b_k' | b_k - b_k'
+        if (row) tb[((it.par ? he : 0) + k) * tc + c] = b;
+    }
     __syncthreads();
     const size_t qstride = (size_t)he * he + (size_t)ho * ho;
-    if (tc == 1 && m0 == 0) {  // the pinned mode alone (the mixed form's launch): one output level per thread
-        for (int z = threadIdx.x; z < nz; z += blockDim.x) {
-            double2 a = make_double2(0.0, 0.0);
-#pragma unroll 4
-            for (int zp = 0; zp < nz; ++zp) {
-                const double2 bb = bpin[zp];
-                const double h1 = __ldg(&ops.PpinT[(size_t)zp * nz + z]);
-                a.x = fma(h1, bb.x, a.x);
-                a.y = fma(h1, bb.y, a.y);
-            }
-            PHI[(size_t)z * g.nm] = a;
-        }
-        return;
-    }
-    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
+    for (int t = threadIdx.x; kLanes == 1 && t < he * tc; t += blockDim.x) {
         const int c = t / he, k = t - c * he;
         const int m = m0 + c;
         if (m >= g.nm || (sp.rhs_only && m != 0)) continue;
@@ -1809,6 +1860,23 @@ __device__ __forceinline__ void pressure_body(GridDev g, Ops ops, StepParams sp,
         }
         PHI[(size_t)k * g.nm + m] = x.a;
         if (k < ho) PHI[(size_t)(nz - 1 - k) * g.nm + m] = x.b;
+    }
+    for (int t0 = 0; kLanes == 2 && t0 < 2 * he * tc; t0 += blockDim.x) {
+        const PairItem<2> it(t0 + threadIdx.x);
+        const int c = it.idx / he, k = it.idx - c * he;
+        const int m = m0 + c, z = it.par ? nz - 1 - k : k;
+        const bool live = c < tc && it.has(k, he, ho) && m < g.nm && !(sp.rhs_only && m != 0);
+        double2 x = make_double2(0.0, 0.0);
+        if (live && m != 0) {
+            const int ky = m / g.nxhp, kx = m - ky * g.nxhp;
+            const double* __restrict__ G = ops.PinvF + (size_t)mode_q(ky, kx, g.ny, g.nxhp) * qstride;
+            x = inv_dot<8>(G + (it.par ? (size_t)he * he : 0) + k, tb + (it.par ? he * tc : 0) + c, it.par ? ho : he,
+                           tc);
+        }
+        x = pair_level(x, it.par);
+        if (!live) continue;
+        if (m == 0) x = inv_dot<8>(ops.PpinT + z, bpin, nz, 1);
+        PHI[(size_t)z * g.nm + m] = x;
     }
 }
 
@@ -2029,12 +2097,13 @@ struct PresRhsTcOp {
     }
 };
 
+template <int kLanes>
 __global__ void __launch_bounds__(256) k_pressure(GridDev g, Ops ops, StepParams sp,
                                                   const double2* __restrict__ US,
                                                   const double2* __restrict__ VS,
                                                   const double2* __restrict__ WS,
                                                   double2* __restrict__ PHI, int tc) {
-    pressure_body(g, ops, sp, US, VS, WS, PHI, tc, blockIdx.x);
+    pressure_body<kLanes>(g, ops, sp, US, VS, WS, PHI, tc, blockIdx.x);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -2219,6 +2288,7 @@ __global__ void k_rk_stage(GridDev g, StepParams sp, double coef, Fields F, Fiel
 // ------------------------------------------------------------------ correction
 // pressure_correction_3d (3D:1903-1929): u = u* - dt grad(phi), p += phi,
 // grad_p_prev = grad(p_total); only its wall planes are consumed (3D:1325-1326).
+template <int kLanes>
 __device__ __forceinline__ void correction_body(GridDev g, Ops ops, StepParams sp,
                                                 const double2* __restrict__ US,
                                                 const double2* __restrict__ VS,
@@ -2234,15 +2304,15 @@ __device__ __forceinline__ void correction_body(GridDev g, Ops ops, StepParams s
     fold_load(tp, PHI, g, m0, tc, he, ho);
     __syncthreads();
     const double dt = sp.dt;
-    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
+    for (int t0 = 0; t0 < kLanes * he * tc; t0 += blockDim.x) {
+        const PairItem<kLanes> it(t0 + threadIdx.x);
+        const int k = it.idx / tc, c = it.idx - k * tc;
         const int m = m0 + c;
-        if (m >= g.nm) continue;
-        const Pair dz = anti_apply(ops.D1e, ops.D1o, tp, k, c, tc, he, ho);
+        const bool live = it.has(k, he, ho) && m < g.nm;
+        const Pair dz = anti_levels<kLanes>(ops.D1e, ops.D1o, tp, k, c, it.par, live, tc, he, ho);
+        if (!live) continue;
         const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
-        const int npt = (k < ho) ? 2 : 1;
-        for (int p = 0; p < npt; ++p) {
-            const int z = p ? nz - 1 - k : k;
+        it.levels(k, ho, nz, [&](int z, int p) {
             const double2 d = p ? dz.b : dz.a;
             const size_t o = (size_t)z * g.nm + m;
             const double2 ph = PHI[o];
@@ -2260,10 +2330,11 @@ __device__ __forceinline__ void correction_body(GridDev g, Ops ops, StepParams s
                 GP[(size_t)wall * g.nm + m] = i_times(mi.ax, pp);
                 GP[(size_t)(2 + wall) * g.nm + m] = i_times(mi.ay, pp);
             }
-        }
+        });
     }
 }
 
+template <int kLanes>
 __global__ void __launch_bounds__(256) k_correction(GridDev g, Ops ops, StepParams sp,
                                                     const double2* __restrict__ US,
                                                     const double2* __restrict__ VS,
@@ -2272,7 +2343,7 @@ __global__ void __launch_bounds__(256) k_correction(GridDev g, Ops ops, StepPara
                                                     double2* __restrict__ U, double2* __restrict__ V,
                                                     double2* __restrict__ W, double2* __restrict__ P,
                                                     double2* __restrict__ GP, int tc) {
-    correction_body(g, ops, sp, US, VS, WS, PHI, U, V, W, P, GP, tc, blockIdx.x);
+    correction_body<kLanes>(g, ops, sp, US, VS, WS, PHI, U, V, W, P, GP, tc, blockIdx.x);
 }
 
 // Wall-plane gradients of p_total alone (used when the state is set).
@@ -3186,23 +3257,81 @@ __global__ void __launch_bounds__(512) k_pressure_mixed(GridDev g, MixedOps mx, 
     pressure_mixed_body<kRefine>(g, mx, ops, sp, US, VS, WS, PHI, PHIZ, tc, blockIdx.x);
 }
 
-// dphi/dz of mode (0,0) in FP64 (one CTA), after k_pressure has written phi.
-__device__ __forceinline__ void dz_mean_mode_body(GridDev g, Ops ops, const double2* __restrict__ PHI,
-                                                  double2* __restrict__ PHIZ, int bx) {
+// The projection of mode (0,0) in FP64, for the mixed form: b = D1.w* scaled as
+// pressure_rhs does, phi = Ppin b, dphi/dz.  One CTA beside the other modes'
+// kernel: three dependent products of nz rows, so four lanes share a row (even
+// and odd part or the halves of the unfolded row, real and imaginary part) and
+// the chains are a quarter as long.  us at nz = 40: 25.6 in two launches with a
+// lane per row, 12.3 now; a mixed 64x48x40 step, which waits for it: 66.6 and
+// 61.4.
+__device__ __forceinline__ double quad_dot(const double* __restrict__ A, int lda, const double* v, int len) {
+    double acc = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < len; ++j) acc = fma(__ldg(&A[(size_t)j * lda]), v[2 * j], acc);
+    return acc;
+}
+
+__device__ __forceinline__ void pressure_mean_body(const GridDev& g, const Ops& ops, const StepParams& sp,
+                                                   const double2* __restrict__ US, const double2* __restrict__ VS,
+                                                   const double2* __restrict__ WS, double2* __restrict__ PHI,
+                                                   double2* __restrict__ PHIZ) {
     extern __shared__ double2 sm[];
-    const int he = ops.he, ho = ops.ho;
-    fold_load(sm, PHI, g, 0, 1, he, ho);
+    const int nz = g.nz, he = ops.he, ho = ops.ho;
+    double2* tile = sm;       // folded w*, then folded phi
+    double2* b = sm + nz;     // right-hand side
+    double2* phi = sm + 2 * nz;
+    const ModeInfo mi = mode_info(g, 0, ops.xw, ops.yw);
+    // y(level of the lane) = A.tile for an antisymmetric operator, component ri
+    auto anti = [&](const double* __restrict__ De, const double* __restrict__ Do, int k, int par, int ri) {
+        double y = 0.0;
+        if (k < (par ? ho : he))
+            y = quad_dot((par ? Do : De) + (size_t)k * (par ? he : ho), 1, &tile[par ? 0 : he].x + ri, par ? he : ho);
+        const double o = __shfl_xor_sync(0xffffffffu, y, 2);
+        return par ? o - y : y + o;
+    };
+    fold_load(tile, WS, g, 0, 1, he, ho);
+    __syncthreads();
+    for (int t0 = 0; t0 < 4 * he; t0 += blockDim.x) {
+        const int t = t0 + threadIdx.x, k = t >> 2, par = (t >> 1) & 1, ri = t & 1;
+        const double d = anti(sp.weak_form ? ops.W1e : ops.D1e, sp.weak_form ? ops.W1o : ops.D1o, k, par, ri);
+        if (k < (par ? ho : he)) {
+            const int z = par ? nz - 1 - k : k;
+            const double2 r = pressure_rhs(g, ops, sp, z, 0, mi, US, VS, make_double2(d, d));
+            (&b[z].x)[ri] = ri ? r.y : r.x;
+        }
+    }
+    __syncthreads();
+    const int nh = (nz + 1) / 2;
+    for (int t0 = 0; t0 < 4 * nz; t0 += blockDim.x) {
+        const int t = t0 + threadIdx.x, z = t >> 2, h = (t >> 1) & 1, ri = t & 1;
+        double y = 0.0;
+        if (z < nz)
+            y = quad_dot(ops.PpinT + (size_t)(h * nh) * nz + z, nz, &b[h * nh].x + ri, h ? nz - nh : nh);
+        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        if (z < nz && h == 0) {
+            (&phi[z].x)[ri] = y;
+            (&PHI[(size_t)z * g.nm].x)[ri] = y;
+        }
+    }
     __syncthreads();
     for (int k = threadIdx.x; k < he; k += blockDim.x) {
-        const Pair d = anti_apply(ops.D1e, ops.D1o, sm, k, 0, 1, he, ho);
-        PHIZ[(size_t)k * g.nm] = d.a;
-        if (k < ho) PHIZ[(size_t)(g.nz - 1 - k) * g.nm] = d.b;
+        const double2 p1 = phi[k], p2 = phi[nz - 1 - k];
+        tile[k] = k < ho ? make_double2(p1.x + p2.x, p1.y + p2.y) : p1;
+        if (k < ho) tile[he + k] = make_double2(p1.x - p2.x, p1.y - p2.y);
+    }
+    __syncthreads();
+    for (int t0 = 0; t0 < 4 * he; t0 += blockDim.x) {
+        const int t = t0 + threadIdx.x, k = t >> 2, par = (t >> 1) & 1, ri = t & 1;
+        const double d = anti(ops.D1e, ops.D1o, k, par, ri);
+        if (k < (par ? ho : he)) (&PHIZ[(size_t)(par ? nz - 1 - k : k) * g.nm].x)[ri] = d;
     }
 }
 
-__global__ void __launch_bounds__(256) k_dz_mean_mode(GridDev g, Ops ops, const double2* __restrict__ PHI,
-                                                      double2* __restrict__ PHIZ) {
-    dz_mean_mode_body(g, ops, PHI, PHIZ, blockIdx.x);
+__global__ void __launch_bounds__(512) k_pressure_mean(GridDev g, Ops ops, StepParams sp,
+                                                       const double2* __restrict__ US, const double2* __restrict__ VS,
+                                                       const double2* __restrict__ WS, double2* __restrict__ PHI,
+                                                       double2* __restrict__ PHIZ) {
+    pressure_mean_body(g, ops, sp, US, VS, WS, PHI, PHIZ);
 }
 
 // Pointwise correction of the mixed form (pressure_correction_3d, 3D:1903-1929)
@@ -3418,14 +3547,6 @@ size_t pressure_mixed_smem(const GridDev& g, int tc) {
            (g.refine ? (size_t)g.nz * tc * sizeof(double2) : 0);  // the FP64 right-hand side kept for the refinement
 }
 
-// Threads of k_vorticity_mixed: as few equal rounds of at most 512 threads as
-// cover its items (256 threads leave a last round of 16 items where an odd
-// he x tc is 2 x 256 + 16, as at nz = 65).  256x256x97: 136 -> 123 us.
-int tile_threads(int items) {
-    const int rounds = std::max(1, (items + 511) / 512);
-    return std::max(64, ((items + rounds - 1) / rounds + 31) / 32 * 32);
-}
-
 namespace {
 
 size_t tile_smem(const GridDev& g, int k, int tc) {
@@ -3471,10 +3592,10 @@ bool tile_fits(const GridDev& g, int k, int tc) {
     if (tc < 1) return false;
     size_t lim = 0;
     switch (k) {
-        case kTileVort: lim = smem_limit(k_vorticity); break;
+        case kTileVort: lim = smem_limit(k_vorticity<1>); break;
         case kTileVisc: lim = smem_limit(k_viscous<double2>); break;
-        case kTilePres: lim = smem_limit(k_pressure); break;
-        case kTileCorr: lim = smem_limit(k_correction); break;
+        case kTilePres: lim = smem_limit(k_pressure<1>); break;
+        case kTileCorr: lim = smem_limit(k_correction<1>); break;
         case kTileDiv: lim = smem_limit(k_divergence); break;
         case kTileVortM: lim = smem_limit(k_vorticity_mixed); break;
         case kTileViscM: lim = smem_limit(k_viscous_mixed); break;
@@ -3486,17 +3607,22 @@ bool tile_fits(const GridDev& g, int k, int tc) {
 
 cudaError_t prepare_step_kernels(const GridDev& g) {
     cudaError_t e;
-    if ((e = set_smem(k_pressure, (2 * (size_t)g.nz + g.nz) * sizeof(double2)))) return e;
-    if ((e = set_smem(k_correction, (size_t)g.nz * sizeof(double2)))) return e;
+    if ((e = set_smem(k_pressure<1>, (2 * (size_t)g.nz + g.nz) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_pressure<2>, (2 * (size_t)g.nz + g.nz) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_correction<1>, (size_t)g.nz * sizeof(double2)))) return e;
+    if ((e = set_smem(k_correction<2>, (size_t)g.nz * sizeof(double2)))) return e;
     if ((e = set_smem(k_pressure_mixed<false>, pressure_mixed_smem(g, tile_cols(g, 2))))) return e;
     if ((e = set_smem(k_pressure_mixed<true>, pressure_mixed_smem(g, tile_cols(g, 2))))) return e;
     if ((e = set_smem(k_viscous<float2>, 6 * (size_t)g.nz * sizeof(double2)))) return e;
     if ((e = set_smem(k_vorticity_mixed, 2 * (size_t)g.nz * tile_cols(g, 1) * sizeof(float2)))) return e;
     if ((e = set_smem(k_viscous_mixed, viscous_mixed_smem(g, tile_cols_mixed(g))))) return e;
-    if ((e = set_smem(k_vorticity, 2 * (size_t)g.nz * tile_cols(g, 2) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_vorticity<1>, 2 * (size_t)g.nz * tile_cols(g, 2) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_vorticity<2>, 2 * (size_t)g.nz * tile_cols(g, 2) * sizeof(double2)))) return e;
     if ((e = set_smem(k_viscous<double2>, 6 * (size_t)g.nz * tile_cols(g, 6) * sizeof(double2)))) return e;
-    if ((e = set_smem(k_pressure, (2 * (size_t)g.nz * tile_cols(g, 2) + g.nz) * sizeof(double2)))) return e;
-    if ((e = set_smem(k_correction, (size_t)g.nz * tile_cols(g, 1) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_pressure<1>, (2 * (size_t)g.nz * tile_cols(g, 2) + g.nz) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_pressure<2>, (2 * (size_t)g.nz * tile_cols(g, 2) + g.nz) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_correction<1>, (size_t)g.nz * tile_cols(g, 1) * sizeof(double2)))) return e;
+    if ((e = set_smem(k_correction<2>, (size_t)g.nz * tile_cols(g, 1) * sizeof(double2)))) return e;
     if ((e = set_smem(k_divergence, (size_t)g.nz * tile_cols(g, 1) * sizeof(double2)))) return e;
     if ((e = set_smem(k_viscous_tc<false>, 0))) return e;
     if ((e = set_smem(k_viscous_tc<true>, 0))) return e;
@@ -3554,11 +3680,29 @@ cudaError_t launch_pi_update(const GridDev& g, const Ops& ops, const PIParams& p
     return cudaGetLastError();
 }
 
+// Threads of a mode-tile kernel with `items` items: as few equal rounds of at
+// most `most` threads as cover them.  A fixed 256 leaves a last round of 16
+// items where an odd he x tc is 2 x 256 + 16 (nz = 65; the mixed vorticity at
+// 256x256x97: 136 -> 123 us), and lanes without an item that keep other CTAs
+// off the SM.
+int tile_threads(int items, int most) {
+    const int rounds = std::max(1, (items + most - 1) / most);
+    return std::max(64, ((items + rounds - 1) / rounds + 31) / 32 * 32);
+}
+
+// Lanes per output pair of the FP64 mode-tile kernels (PairItem): two where one
+// per pair gives every SM less than 7 warps.  us per step, one and two lanes:
+// 32x32x17 64 and 53, 32x32x33 80 and 65, 64x48x40 120 and 113; past the line
+// 64x64x33 115 and 116, 96x64x33 154 and 160, 96x96x33 203 and 210.
+int pair_lanes(const GridDev& g) { return (long long)g.nm * (g.nz - g.nz / 2) < 152LL * 224 ? 2 : 1; }
+
 cudaError_t launch_vorticity(const GridDev& g, const Ops& ops, const double2* U, const double2* V,
                              const double2* W, double2* OX, double2* OY, double2* OZ, cudaStream_t s) {
     const int tc = tile_width(g, kTileVort);
     const size_t sm = 2 * (size_t)g.nz * tc * sizeof(double2);
-    k_vorticity<<<(g.nm + tc - 1) / tc, 256, sm, s>>>(g, ops, U, V, W, OX, OY, OZ, tc);
+    const int lanes = pair_lanes(g), nt = tile_threads(lanes * (g.nz - g.nz / 2) * tc, 256);
+    auto k = lanes == 2 ? k_vorticity<2> : k_vorticity<1>;
+    k<<<(g.nm + tc - 1) / tc, nt, sm, s>>>(g, ops, U, V, W, OX, OY, OZ, tc);
     return cudaGetLastError();
 }
 
@@ -3700,16 +3844,15 @@ cudaError_t launch_vorticity_mixed(const GridDev& g, const MixedOps& mx, const O
                                    const double2* V, const double2* W, FFields out, cudaStream_t s) {
     const int tc = tile_width(g, kTileVortM);
     const size_t sm = 2 * (size_t)g.nz * tc * sizeof(float2);
-    k_vorticity_mixed<<<(g.nm + tc - 1) / tc, tile_threads((g.nz - g.nz / 2) * tc), sm, s>>>(g, mx, ops, U, V, W, out, tc);
+    k_vorticity_mixed<<<(g.nm + tc - 1) / tc, tile_threads((g.nz - g.nz / 2) * tc, 512), sm, s>>>(g, mx, ops, U, V, W, out, tc);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pressure_mean_mode(const GridDev& g, const Ops& ops, const StepParams& sp, const double2* US,
                                       const double2* VS, const double2* WS, double2* PHI, double2* PHIZ,
                                       cudaStream_t s) {
-    // mode (0,0) of the mixed form in FP64: pinned Poisson, then its dphi/dz
-    k_pressure<<<1, 256, (2 * (size_t)g.nz + g.nz) * sizeof(double2), s>>>(g, ops, sp, US, VS, WS, PHI, 1);
-    k_dz_mean_mode<<<1, 64, (size_t)g.nz * sizeof(double2), s>>>(g, ops, PHI, PHIZ);
+    const int nt = std::min(512, (4 * g.nz + 31) / 32 * 32);
+    k_pressure_mean<<<1, nt, 3 * (size_t)g.nz * sizeof(double2), s>>>(g, ops, sp, US, VS, WS, PHI, PHIZ);
     return cudaGetLastError();
 }
 
@@ -3771,7 +3914,9 @@ cudaError_t launch_pressure(const GridDev& g, const Ops& ops, const StepParams& 
                             const double2* VS, const double2* WS, double2* PHI, cudaStream_t s) {
     const int tc = tile_width(g, kTilePres);
     const size_t sm = (2 * (size_t)g.nz * tc + g.nz) * sizeof(double2);
-    k_pressure<<<(g.nm + tc - 1) / tc, 256, sm, s>>>(g, ops, sp, US, VS, WS, PHI, tc);
+    const int lanes = pair_lanes(g), nt = tile_threads(lanes * (g.nz - g.nz / 2) * tc, 256);
+    auto k = lanes == 2 ? k_pressure<2> : k_pressure<1>;
+    k<<<(g.nm + tc - 1) / tc, nt, sm, s>>>(g, ops, sp, US, VS, WS, PHI, tc);
     return cudaGetLastError();
 }
 
@@ -3780,7 +3925,9 @@ cudaError_t launch_correction(const GridDev& g, const Ops& ops, const StepParams
                               double2* V, double2* W, double2* P, double2* GP, cudaStream_t s) {
     const int tc = tile_width(g, kTileCorr);
     const size_t sm = (size_t)g.nz * tc * sizeof(double2);
-    k_correction<<<(g.nm + tc - 1) / tc, 256, sm, s>>>(g, ops, sp, US, VS, WS, PHI, U, V, W, P, GP, tc);
+    const int lanes = pair_lanes(g), nt = tile_threads(lanes * (g.nz - g.nz / 2) * tc, 256);
+    auto k = lanes == 2 ? k_correction<2> : k_correction<1>;
+    k<<<(g.nm + tc - 1) / tc, nt, sm, s>>>(g, ops, sp, US, VS, WS, PHI, U, V, W, P, GP, tc);
     return cudaGetLastError();
 }
 
@@ -3900,7 +4047,7 @@ struct RsPi {
 struct RsVort64 {
     static constexpr int kMinCtas = 2;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        vorticity_body(d.g, d.ops, d.U, d.V, d.W, d.US, d.VS, d.WS, d.g.tc[kTileVort], b);
+        vorticity_body<1>(d.g, d.ops, d.U, d.V, d.W, d.US, d.VS, d.WS, d.g.tc[kTileVort], b);
     }
 };
 
@@ -3969,7 +4116,7 @@ struct RsViscMean {
 struct RsPres64 {
     static constexpr int kMinCtas = 4;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        pressure_body(d.g, d.ops, d.sp, d.US, d.VS, d.WS, d.PHI, d.g.tc[kTilePres], b);
+        pressure_body<1>(d.g, d.ops, d.sp, d.US, d.VS, d.WS, d.PHI, d.g.tc[kTilePres], b);
     }
 };
 
@@ -4003,16 +4150,14 @@ struct RsPres32 {
 struct RsPresMean {
     static constexpr int kMinCtas = 1;
     static __device__ __forceinline__ void run(const RunDesc& d, int) {
-        pressure_body(d.g, d.ops, d.sp, d.US, d.VS, d.WS, d.PHI, 1, 0);
-        __syncthreads();  // phi of mode (0,0) written by this CTA
-        dz_mean_mode_body(d.g, d.ops, d.PHI, d.PHIZ, 0);
+        pressure_mean_body(d.g, d.ops, d.sp, d.US, d.VS, d.WS, d.PHI, d.PHIZ);
     }
 };
 
 struct RsCorr64 {
     static constexpr int kMinCtas = 4;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        correction_body(d.g, d.ops, d.sp, d.US, d.VS, d.WS, d.PHI, d.U, d.V, d.W, d.P, d.GP, d.g.tc[kTileCorr], b);
+        correction_body<1>(d.g, d.ops, d.sp, d.US, d.VS, d.WS, d.PHI, d.U, d.V, d.W, d.P, d.GP, d.g.tc[kTileCorr], b);
     }
 };
 
