@@ -207,8 +207,8 @@ struct Ops {
     double* yw;      // [ny]
     double* ksq;     // xsq+ysq per unique q     [nq]
     double* S;       // stiffness (2/ybar) sum_m d1(m,k) d1(m,n) zwts(m), [nz][nz] (jacgs)
-    double* HinvF;   // folded Helmholtz inverses      [nq][he*he + ho*ho]
-    double* PinvF;   // folded Poisson inverses        [nq][he*he + ho*ho]
+    double* HinvF;   // folded Helmholtz inverses      [nq][he*he + ho*ho] (mixed: q = 0 only)
+    double* PinvF;   // folded Poisson inverses        [nq][he*he + ho*ho] (mixed: none read)
     double* PpinT;   // pinned (0,0) Poisson inverse, unfolded, transposed [nz][nz]
     // PinvF in 58-bit fixed point for the solve on the integer pipes (FP64
     // runs with the tensor-core forms), or null: entry (j, k) of a folded
