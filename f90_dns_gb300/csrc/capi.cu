@@ -66,6 +66,8 @@ struct dns3d_handle {
     int red_blocks = 0;
     std::vector<double> zpts, zwts;
     std::vector<void*> allocs;
+    char* slab = nullptr;  // rest of the last allocation dev_alloc made
+    size_t slab_left = 0;
     int step = 0;
     double time = 0.0;
     cudaGraphExec_t graph = nullptr;
@@ -102,24 +104,41 @@ int cuda_fail(dns3d_handle* h, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail((h), e_, #call); \
     } while (0)
 
-template <typename T>
-int dev_alloc(dns3d_handle* h, T** p, size_t count) {
-    void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, count * sizeof(T) > 0 ? count * sizeof(T) : 1);
-    if (e != cudaSuccess) return cuda_fail(h, e, "cudaMalloc");
-    h->allocs.push_back(q);
-    // every buffer starts zeroed (work buffers are read by the tile autotuner)
-    e = h->stream ? cudaMemsetAsync(q, 0, count * sizeof(T), h->stream) : cudaMemset(q, 0, count * sizeof(T));
-    if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemset");
-    *p = static_cast<T*>(q);
-    return DNS3D_OK;
-}
-
 size_t spec_elems(const dns3d_config& c) { return (size_t)(c.nx / 2 + 1) * c.ny * c.nz; }
 size_t phys_elems(const dns3d_config& c) { return (size_t)c.nx * c.ny * c.nz; }
 int n_unique_q(const dns3d_config& c) { return (c.ny / 2 + 1) * (c.nx / 2 + 1); }
 // k^2 values whose Helmholtz and Poisson inverses a handle builds
 int n_inverses(const dns3d_config& c) { return c.precision == DNS3D_PREC_MIXED ? 2 : n_unique_q(c); }
+
+size_t footprint(const dns3d_config& c);
+constexpr size_t kTableBytes = 16ull << 20;  // footprint's allowance for operators, tables, reductions
+
+// Device memory from one allocation of the handle's size, made by the first
+// call, and from blocks of 4 MB for what exceeds it (256-byte steps; freed with
+// the handle).  A buffer each cost a handle 1.8 ms of cudaMalloc and 0.8 ms of
+// cudaFree (96x96x65, mixed; creating it 5.6 and 3.9 ms, six handles of serving
+// grids freed in 5.0 and 1.0 ms).  Every buffer starts zeroed (work
+// buffers are read by the tile autotuner).
+template <typename T>
+int dev_alloc(dns3d_handle* h, T** p, size_t count) {
+    constexpr size_t kBlock = 4ull << 20;
+    const size_t need = (std::max<size_t>(count * sizeof(T), 1) + 255) / 256 * 256;
+    if (need > h->slab_left) {
+        const size_t block = std::max(need, h->allocs.empty() ? footprint(h->cfg) - kTableBytes + kBlock : kBlock);
+        void* q = nullptr;
+        cudaError_t e = cudaMalloc(&q, block);
+        if (e != cudaSuccess) return cuda_fail(h, e, "cudaMalloc");
+        h->allocs.push_back(q);
+        e = h->stream ? cudaMemsetAsync(q, 0, block, h->stream) : cudaMemset(q, 0, block);
+        if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemset");
+        h->slab = static_cast<char*>(q);
+        h->slab_left = block;
+    }
+    *p = reinterpret_cast<T*>(h->slab);
+    h->slab += need;
+    h->slab_left -= need;
+    return DNS3D_OK;
+}
 
 int validate(const dns3d_config* c) {
     if (!c) return DNS3D_E_INVALID;
@@ -594,6 +613,39 @@ int run_step_body(dns3d_handle* h) {
     return run_correction(h, true);
 }
 
+size_t footprint(const dns3d_config& c) {
+    const size_t se = spec_elems(c), pe = phys_elems(c);
+    const size_t nm = (size_t)(c.nx / 2 + 1) * c.ny;
+    const size_t nq = (size_t)n_unique_q(c);
+    const size_t nz2 = (size_t)c.nz * c.nz;
+    size_t b = 0;
+    b += 11 * se * sizeof(double2);          // U V W P SU SV SW US VS WS PHI
+    if (c.convection_scheme == 1) b += 3 * se * sizeof(double2);  // jst4 stage state
+    b += 4 * nm * sizeof(double2);           // GP
+    b += 6 * se * sizeof(double2);           // FFT scratch
+    b += 6 * pe * sizeof(double);            // physical fields
+    const size_t hz = (size_t)c.nz / 2, ez = (size_t)c.nz - hz;
+    b += (2 * (size_t)n_inverses(c) * (ez * ez + hz * hz) + 2 * nz2) * sizeof(double);  // folded inverses, pinned, S
+    if (c.precision == DNS3D_PREC_MIXED)
+        // FP32 spectra, sources and scratch, dphi/dz (and the physical planes
+        // without compile-time transforms)
+        b += (6 + 3 + 6) * se * sizeof(float2) + se * sizeof(double2) +
+             (fft_ct_supported(c.ny, c.nx / 2) ? 0 : 6 * pe * sizeof(float));
+    else {
+        if (fft_ct_supported(c.ny, c.nx / 2))  // exponents of the nonlinear term's integer spectra
+            b += ((size_t)6 * (c.nx / 2 + 1) + (size_t)3 * c.ny) * c.nz * sizeof(int);
+    }
+    if (c.precision != DNS3D_PREC_MIXED && tc_supported(c.nz)) {
+        const TcGeom t = tc_geom(c.nz);
+        if (c.use_crank_nicolson && c.linear_solver == 0)  // digit slices of the Helmholtz inverses
+            b += nq * (tc_q_halves(t) * sizeof(__half) + (size_t)t.m8 * sizeof(int));
+        b += (size_t)kTcSlices * tc_blocks(t, true).a * sizeof(__half);  // digit image of D1
+        if (!c.use_weak_form_divergence)  // fixed-point Poisson inverses and row exponents
+            b += nq * (fx_qstride((int)ez, (int)hz) * sizeof(long long) + (size_t)c.nz * sizeof(int));
+    }
+    return b + kTableBytes;
+}
+
 void release(dns3d_handle* h) {
     if (!h) return;
     if (h->graph) cudaGraphExecDestroy(h->graph);
@@ -657,37 +709,7 @@ int dns3d_config_read_namelist(const char* path, dns3d_config* cfg) {
 
 int dns3d_footprint_bytes(const dns3d_config* c, unsigned long long* bytes) {
     if (!c || !bytes) return DNS3D_E_INVALID;
-    const size_t se = spec_elems(*c), pe = phys_elems(*c);
-    const size_t nm = (size_t)(c->nx / 2 + 1) * c->ny;
-    const size_t nq = (size_t)n_unique_q(*c);
-    const size_t nz2 = (size_t)c->nz * c->nz;
-    size_t b = 0;
-    b += 11 * se * sizeof(double2);          // U V W P SU SV SW US VS WS PHI
-    if (c->convection_scheme == 1) b += 3 * se * sizeof(double2);  // jst4 stage state
-    b += 4 * nm * sizeof(double2);           // GP
-    b += 6 * se * sizeof(double2);           // FFT scratch
-    b += 6 * pe * sizeof(double);            // physical fields
-    const size_t hz = (size_t)c->nz / 2, ez = (size_t)c->nz - hz;
-    b += (2 * (size_t)n_inverses(*c) * (ez * ez + hz * hz) + 2 * nz2) * sizeof(double);  // folded inverses, pinned, S
-    if (c->precision == DNS3D_PREC_MIXED)
-        // FP32 spectra, sources and scratch, dphi/dz (and the physical planes
-        // without compile-time transforms)
-        b += (6 + 3 + 6) * se * sizeof(float2) + se * sizeof(double2) +
-             (fft_ct_supported(c->ny, c->nx / 2) ? 0 : 6 * pe * sizeof(float));
-    else {
-        if (fft_ct_supported(c->ny, c->nx / 2))  // exponents of the nonlinear term's integer spectra
-            b += ((size_t)6 * (c->nx / 2 + 1) + (size_t)3 * c->ny) * c->nz * sizeof(int);
-    }
-    if (c->precision != DNS3D_PREC_MIXED && tc_supported(c->nz)) {
-        const TcGeom t = tc_geom(c->nz);
-        if (c->use_crank_nicolson && c->linear_solver == 0)  // digit slices of the Helmholtz inverses
-            b += nq * (tc_q_halves(t) * sizeof(__half) + (size_t)t.m8 * sizeof(int));
-        b += (size_t)kTcSlices * tc_blocks(t, true).a * sizeof(__half);  // digit image of D1
-        if (!c->use_weak_form_divergence)  // fixed-point Poisson inverses and row exponents
-            b += nq * (fx_qstride((int)ez, (int)hz) * sizeof(long long) + (size_t)c->nz * sizeof(int));
-    }
-    b += 16ull << 20;                        // operators, tables, reductions
-    *bytes = b;
+    *bytes = footprint(*c);
     return DNS3D_OK;
 }
 
@@ -962,19 +984,14 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     lgl_nodes_weights(nz, h->zpts, h->zwts);
     lgl_diff_matrix(h->zpts, c.lgl_dmatrix_guard != 0, d1);
     for (int i = 0; i < nz; ++i)  // d2 = matmul(d1, d1) (3D:801)
-        for (int j = 0; j < nz; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < nz; ++k) s += d1[(size_t)i * nz + k] * d1[(size_t)k * nz + j];
-            d2[(size_t)i * nz + j] = s;
-        }
+        for (int k = 0; k < nz; ++k)
+            for (int j = 0; j < nz; ++j) d2[(size_t)i * nz + j] += d1[(size_t)i * nz + k] * d1[(size_t)k * nz + j];
     // stiffness S_kn = sum_m d1(m,k) d1(m,n) zwts(m) (2/ybar)  (3D:1467-1471)
-    std::vector<double> S((size_t)nz * nz);
-    for (int k = 0; k < nz; ++k)
-        for (int n = 0; n < nz; ++n) {
-            double s = 0.0;
-            for (int m = 0; m < nz; ++m) s += d1[(size_t)m * nz + k] * d1[(size_t)m * nz + n] * h->zwts[m];
-            S[(size_t)k * nz + n] = s * (2.0 / ybar);
-        }
+    std::vector<double> S((size_t)nz * nz, 0.0);
+    for (int m = 0; m < nz; ++m)
+        for (int k = 0; k < nz; ++k)
+            for (int n = 0; n < nz; ++n) S[(size_t)k * nz + n] += d1[(size_t)m * nz + k] * d1[(size_t)m * nz + n] * h->zwts[m];
+    for (double& v : S) v *= 2.0 / ybar;
     const double theta = c.use_crank_nicolson ? 0.5 : 1.0;
     const double helm_f = theta * c.dt / c.re;
     std::vector<double> D1s((size_t)nz * nz), D2s((size_t)nz * nz), wh(nz), S0(nz), Sn(nz),

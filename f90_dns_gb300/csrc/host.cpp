@@ -107,8 +107,8 @@ void lgl_diff_matrix(const std::vector<double>& x, bool guard, std::vector<doubl
 
 // Cyclic Jacobi rotations until the off-diagonal mass is at rounding level.
 void jacobi_eigen(int n, std::vector<double>& a, std::vector<double>& w, std::vector<double>& y) {
-    y.assign((size_t)n * n, 0.0);
-    for (int i = 0; i < n; ++i) y[(size_t)i * n + i] = 1.0;
+    std::vector<double> yt((size_t)n * n, 0.0);  // eigenvectors as rows
+    for (int i = 0; i < n; ++i) yt[(size_t)i * n + i] = 1.0;
     auto A = [&](int i, int j) -> double& { return a[(size_t)i * n + j]; };
     double diag2 = 0.0;
     for (int i = 0; i < n; ++i) diag2 += A(i, i) * A(i, i);
@@ -129,15 +129,14 @@ void jacobi_eigen(int n, std::vector<double>& a, std::vector<double>& w, std::ve
                     A(k, p) = c * akp - s * akq;
                     A(k, q) = s * akp + c * akq;
                 }
-                for (int k = 0; k < n; ++k) {
-                    const double apk = A(p, k), aqk = A(q, k);
-                    A(p, k) = c * apk - s * aqk;
-                    A(q, k) = s * apk + c * aqk;
-                }
-                for (int k = 0; k < n; ++k) {
-                    const double ykp = y[(size_t)k * n + p], ykq = y[(size_t)k * n + q];
-                    y[(size_t)k * n + p] = c * ykp - s * ykq;
-                    y[(size_t)k * n + q] = s * ykp + c * ykq;
+                for (std::vector<double>* m : {&a, &yt}) {
+                    double* __restrict__ rp = m->data() + (size_t)p * n;
+                    double* __restrict__ rq = m->data() + (size_t)q * n;
+                    for (int k = 0; k < n; ++k) {
+                        const double vp = rp[k], vq = rq[k];
+                        rp[k] = c * vp - s * vq;
+                        rq[k] = s * vp + c * vq;
+                    }
                 }
             }
         }
@@ -147,12 +146,11 @@ void jacobi_eigen(int n, std::vector<double>& a, std::vector<double>& w, std::ve
     for (int i = 0; i < n; ++i) idx[i] = i;
     std::sort(idx.begin(), idx.end(), [&](int i, int j) { return A(i, i) < A(j, j); });
     w.resize(n);
-    std::vector<double> ys((size_t)n * n);
+    y.resize((size_t)n * n);
     for (int c = 0; c < n; ++c) {
         w[c] = A(idx[c], idx[c]);
-        for (int r = 0; r < n; ++r) ys[(size_t)r * n + c] = y[(size_t)r * n + idx[c]];
+        for (int r = 0; r < n; ++r) y[(size_t)r * n + c] = yt[(size_t)idx[c] * n + r];
     }
-    y.swap(ys);
 }
 
 // ------------------------------------------------------------------ namelist
