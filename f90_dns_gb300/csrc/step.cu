@@ -2534,7 +2534,7 @@ __global__ void k_products32(FRFields in, FRFields out, size_t n) {
 // advanced in FP64 by k_viscous.
 __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops ops, StepParams sp,
                                                    Fields F, FFields Src, const double2* __restrict__ GP,
-                                                   Fields Out, int tc, int bx, bool stage_mats = true) {
+                                                   Fields Out, int tc, int bx, int c0, int c1, bool stage_mats) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int hei = mx.hei, hoi = mx.hoi, pe4 = mx.pe4, po4 = mx.po4;
     const int nr = pe4 + po4;        // folded rows (even block, then odd block)
@@ -2561,7 +2561,7 @@ __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops o
         for (int t = threadIdx.x; t < hoi * (po4 / 4); t += blockDim.x) sBo[t] = __ldg(&A[t]);
     }
     const float dt = d2f(sp.dt), cf = d2f(sp.cn_fac), ff = d2f(sp.helm_f);
-    for (int comp = 0; comp < 3; ++comp) {
+    for (int comp = c0; comp < c1; ++comp) {
         // fold the interior column: even rows k < hei, odd rows pe4 + k
         for (int t = threadIdx.x; t < pe4 * tc; t += blockDim.x) {
             const int k = tile_row(td, t), c = t - k * tc;
@@ -2729,14 +2729,19 @@ __device__ __forceinline__ void viscous_mixed_body(GridDev g, MixedOps mx, Ops o
     }
 }
 
-// Persistent: a CTA stages the matrices once and takes every gridDim.x-th tile.
+// Persistent: a CTA stages the matrices once and takes every gridDim.x-th
+// (component, tile), the tiles of a component in order.  On a small grid the
+// components run side by side instead of one after the other in each CTA, which
+// waits for loads and barriers most of the time (us with all three in a CTA and
+// now: 64x48x40 24.6 and 14.3, 96x96x49 30.5 and 22.5, 128x128x65 51 and 45,
+// 256x256x97 301 and 289).
 __global__ void __launch_bounds__(256) k_viscous_mixed(GridDev g, MixedOps mx, Ops ops, StepParams sp,
                                                        Fields F, FFields Src, const double2* __restrict__ GP,
                                                        Fields Out, int tc) {
     const int ntiles = (g.nm + tc - 1) / tc;
-    for (int bx = blockIdx.x; bx < ntiles; bx += gridDim.x) {
-        viscous_mixed_body(g, mx, ops, sp, F, Src, GP, Out, tc, bx, bx == (int)blockIdx.x);
-        __syncthreads();  // the tile buffers are reused by the next tile
+    for (int u = blockIdx.x; u < 3 * ntiles; u += gridDim.x) {
+        const int comp = u / ntiles;
+        viscous_mixed_body(g, mx, ops, sp, F, Src, GP, Out, tc, u - comp * ntiles, comp, comp + 1, u == (int)blockIdx.x);
     }
 }
 
@@ -3901,11 +3906,13 @@ cudaError_t launch_viscous_mixed(const GridDev& g, const MixedOps& mx, const Ops
                                  Fields F, FFields Src, const double2* GP, Fields Out, cudaStream_t s) {
     const int tc = tile_width(g, kTileViscM);
     const size_t sm = viscous_mixed_smem(g, tc);
-    const int ntiles = (g.nm + tc - 1) / tc;
+    const int units = 3 * ((g.nm + tc - 1) / tc);
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_viscous_mixed, 256, sm);
     if (e) return e;
-    const int nb = std::min(ntiles, std::max(1, per_sm) * num_sms());
+    // one CTA's place stays free for the (0,0) mode's kernel beside this one, which
+    // would run after it (128x128x65: 178 and 168 us per step)
+    const int nb = std::min(units, std::max(1, per_sm * num_sms() - 1));
     k_viscous_mixed<<<nb, 256, sm, s>>>(g, mx, ops, sp, F, Src, GP, Out, tc);
     return cudaGetLastError();
 }
@@ -4101,7 +4108,7 @@ struct RsVisc32 {
     static constexpr int kMinCtas = 4;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
         viscous_mixed_body(d.g, d.mx, d.ops, d.sp, fields3(d.U, d.V, d.W), desc_fields<float2, 3>(d.src), d.GP,
-                           fields3(d.US, d.VS, d.WS), d.g.tc[kTileViscM], b);
+                           fields3(d.US, d.VS, d.WS), d.g.tc[kTileViscM], b, 0, 3, true);
     }
 };
 
