@@ -1923,59 +1923,71 @@ __device__ __forceinline__ int4 fx_limbs(long long re, long long im) {
     return make_int4((int)(re & 0x7FFFFFF), (int)(re >> 27), (int)(im & 0x7FFFFFF), (int)(im >> 27));
 }
 
-// Modes per CTA of the solve: their fixed-point inverses are staged in shared
-// memory (at most 64 KB of them, at least one mode), and one thread takes one
-// folded row of one mode (at most 512 rows).
-__host__ __device__ inline int fx_solve_modes(int nz) {
+// Operators per CTA of the solve: they are staged in shared memory, each for
+// its two modes (kx, +-ky), and two lanes take one folded row pair of one mode
+// (at most 288 threads, the 260 of nz = 129: four CTAs of 56 registers fit an SM).
+constexpr int kFxSolveThreads = 288;
+__host__ __device__ inline int fx_solve_ops(int nz) {
     const int ho = nz / 2, he = nz - ho;
     int t = (int)(65536 / (fx_qstride(he, ho) * sizeof(long long)));
-    if (t * nz > 512) t = 512 / nz;
+    if (4 * t * he > kFxSolveThreads) t = kFxSolveThreads / (4 * he);
     return t < 1 ? 1 : t;
 }
-__host__ __device__ inline int fx_solve_threads(int nz) { return (nz * fx_solve_modes(nz) + 31) / 32 * 32; }
+__host__ __device__ inline int fx_solve_threads(int nz) {
+    return (4 * (nz - nz / 2) * fx_solve_ops(nz) + 31) / 32 * 32;
+}
 __host__ __device__ inline size_t fx_solve_smem(int nz) {
-    const int ho = nz / 2, he = nz - ho, tc = fx_solve_modes(nz);
-    return (size_t)tc * fx_qstride(he, ho) * sizeof(long long) + (2 * (size_t)nz * tc + nz) * sizeof(double2) +
-           (size_t)tc * sizeof(int);
+    const int ho = nz / 2, he = nz - ho, tq = fx_solve_ops(nz);
+    return (size_t)tq * (fx_qstride(he, ho) * sizeof(long long) + 2 * (size_t)nz * sizeof(double2) + 4 * sizeof(int));
 }
 
 // The Poisson solve of pressure_body for a right-hand side already in PHI
-// (unfolded, as pressure_body forms it), fx_solve_modes(nz) modes from
-// bx tc: the modes' fixed-point inverses are copied into shared memory with
-// cp.async (16-byte pieces, all in flight at once) while the CTA stages the
-// unfolded columns, takes each column's power of two and folds it in fixed
-// point; then each thread applies one folded row (above; the pinned mode
-// (0,0) unfolded, with its FP64 inverse), and the results are unfolded over
-// the right-hand side.  A CTA reads its tile whole before it writes, so the
+// (unfolded, as pressure_body forms it), the modes of fx_solve_ops(nz) operators
+// q from bx fx_solve_ops(nz): the fixed-point inverses are copied into shared
+// memory with cp.async (16-byte pieces, all in flight at once) while the CTA
+// stages the unfolded columns, takes each column's power of two and folds it in
+// place in fixed point; then two lanes apply the even and the odd row of an
+// output pair (above; the pinned mode (0,0) unfolded, with its FP64 inverse) and
+// exchange the results.  A CTA reads its columns whole before it writes, so the
 // solve is in place.  A column with a non-finite entry gets NaN throughout.
+// An operator staged for one mode at a time (twice read; its columns, folded
+// columns and results in three buffers) left 15 to 21 warps on an SM waiting for
+// the operators; now 27 to 36.  With the right-hand side's kernel before it, in
+// us: 128x128x65 115 and 100, 96x192x81 188 and 164, 512x384x129 3330 and 2710.
 __device__ __forceinline__ void pressure_solve_body(const GridDev& g, const Ops& ops, double2* __restrict__ PHI,
                                                     int bx) {
     extern __shared__ __align__(16) unsigned char smc[];
     const int nz = g.nz, he = ops.he, ho = ops.ho;
-    const int tc = fx_solve_modes(nz), tsz = nz * tc;
+    const int tq = fx_solve_ops(nz), tc = 2 * tq, tsz = nz * tc;  // columns: tq of ky >= 0, tq of -ky
     const size_t qs = fx_qstride(he, ho);
-    long long* sG = reinterpret_cast<long long*>(smc);                  // inverses of the tile's modes [tc][qs]
-    double2* su = reinterpret_cast<double2*>(sG + (size_t)tc * qs);   // unfolded columns [nz][tc], then results
-    int4* tb = reinterpret_cast<int4*>(su + tsz);                      // folded columns in fixed point (limbs)
-    double2* bpin = su + 2 * tsz;                                      // unfolded rhs of mode (0,0)
-    int* sF = reinterpret_cast<int*>(bpin + nz);                       // column exponents
-    const int m0 = bx * tc;
+    long long* sG = reinterpret_cast<long long*>(smc);                  // the operators [tq][qs]
+    double2* bpin = reinterpret_cast<double2*>(sG);                     // q = 0: unfolded rhs of mode (0,0) instead
+    double2* su = reinterpret_cast<double2*>(sG + (size_t)tq * qs);   // unfolded columns [nz][tc], then
+    int4* tb = reinterpret_cast<int4*>(su);                            // folded ones (limbs): even row k at k, odd at nz-1-k
+    int* sF = reinterpret_cast<int*>(su + tsz);                        // column exponents
+    int* sM = sF + tc;                                                 // the columns' modes (-1: none)
+    const int q0 = bx * tq;
     {
-        const int n16 = (int)(qs / 2);  // 16-byte pieces per mode
-        for (int c = 0; c < tc; ++c) {
-            const int m = m0 + c;
-            if (m >= g.nm || m == 0) continue;
-            const int ky = m / g.nxhp, kx = m - ky * g.nxhp;
-            const long long* src = ops.PinvI + (size_t)mode_q(ky, kx, g.ny, g.nxhp) * qs;
+        const int n16 = (int)(qs / 2);  // 16-byte pieces per operator
+        for (int c = q0 == 0 ? 1 : 0; c < tq && q0 + c < ops.nq; ++c) {
+            const long long* src = ops.PinvI + (size_t)(q0 + c) * qs;
             long long* dst = sG + (size_t)c * qs;
             for (int i = threadIdx.x; i < n16; i += blockDim.x) cp_async16(dst + 2 * i, src + 2 * i);
         }
         cp_async_commit();
     }
+    for (int c = threadIdx.x; c < tc; c += blockDim.x) {
+        const int q = q0 + (c < tq ? c : c - tq);
+        const int ka = q / g.nxhp, kx = q - ka * g.nxhp;
+        int m = -1;
+        if (q < ops.nq && (c < tq || (ka != 0 && 2 * ka != g.ny))) m = (c < tq ? ka : g.ny - ka) * g.nxhp + kx;
+        sM[c] = m;
+    }
+    __syncthreads();
     for (int t = threadIdx.x; t < tsz; t += blockDim.x) {
         const int z = t / tc, c = t - z * tc;
-        const int m = m0 + c;
-        const double2 v = m < g.nm ? PHI[(size_t)z * g.nm + m] : make_double2(0.0, 0.0);
+        const int m = sM[c];
+        const double2 v = m >= 0 ? PHI[(size_t)z * g.nm + m] : make_double2(0.0, 0.0);
         su[t] = v;
         if (m == 0) bpin[z] = v;
     }
@@ -2011,72 +2023,51 @@ __device__ __forceinline__ void pressure_solve_body(const GridDev& g, const Ops&
             const double2 b = su[(nz - 1 - k) * tc + c];
             const long long bx2 = tc_fixed(b.x, f), by = tc_fixed(b.y, f);
             tb[k * tc + c] = fx_limbs(ax + bx2, ay + by);
-            tb[(he + k) * tc + c] = fx_limbs(ax - bx2, ay - by);
+            tb[(nz - 1 - k) * tc + c] = fx_limbs(ax - bx2, ay - by);
         } else {
             tb[k * tc + c] = fx_limbs(ax, ay);
         }
     }
     cp_async_wait_all();
     __syncthreads();  // the folded tile and every thread's operator pieces
-    // one folded row r of one column per thread (rows of a column on adjacent lanes)
-    for (int t = threadIdx.x; t < tsz; t += blockDim.x) {
-        const int c = t / nz, r = t - c * nz;
-        const int m = m0 + c;
-        if (m >= g.nm) continue;
-        if (m == 0) {  // the pinned mode: output level r, unfolded, FP64
-            double2 a = make_double2(0.0, 0.0);
-            for (int zp = 0; zp < nz; ++zp) {
-                const double2 bb = bpin[zp];
-                const double h1 = __ldg(&ops.PpinT[(size_t)zp * nz + r]);
-                a.x = fma(h1, bb.x, a.x);
-                a.y = fma(h1, bb.y, a.y);
-            }
-            PHI[(size_t)r * g.nm] = a;
-            continue;
-        }
-        const int f = sF[c];
-        double2 x;
-        if (f == INT_MIN) {
-            x.x = x.y = __longlong_as_double(0x7FF8000000000000LL);
-        } else {
-            const int ky = m / g.nxhp, kx = m - ky * g.nxhp;
-            const size_t q = (size_t)mode_q(ky, kx, g.ny, g.nxhp);
-            const bool even = r < he;
-            const int n = even ? he : ho, k = even ? r : r - he;
-            const long long* G = sG + (size_t)c * qs + (even ? 0 : (size_t)he * he) + k;
-            const int4* bcol = tb + (even ? 0 : he * tc) + c;
-            FxAcc sx{}, sy{};
+    // rows of a column on adjacent lane pairs
+    for (int t0 = 0; t0 < 2 * he * tc; t0 += blockDim.x) {
+        const PairItem<2> it(t0 + threadIdx.x);
+        const int par = it.par, c = it.idx / he, k = it.idx - c * he;
+        const int m = c < tc ? sM[c] : -1;
+        const bool live = m >= 0 && it.has(k, he, ho);
+        double2 x = make_double2(0.0, 0.0);
+        if (live && m != 0) {
+            const int f = sF[c];
+            if (f == INT_MIN) {
+                x.x = x.y = __longlong_as_double(0x7FF8000000000000LL);
+            } else {
+                const int cq = c < tq ? c : c - tq, n = par ? ho : he;
+                const long long* G = sG + (size_t)cq * qs + (par ? (size_t)he * he : 0) + k;
+                const int4* bcol = tb + (par ? (nz - 1) * tc : 0) + c;
+                const int step = par ? -tc : tc;
+                FxAcc sx{}, sy{};
 #pragma unroll 4
-            for (int j = 0; j < n; ++j, G += n, bcol += tc) {
-                const long long a = *G;
-                const int a0 = (int)(a & 0x1FFFFFFF), a1 = (int)(a >> 29);
-                const int4 b = *bcol;
-                fx_mac(sx, a0, a1, b.x, b.y);
-                fx_mac(sy, a0, a1, b.z, b.w);
+                for (int j = 0; j < n; ++j, G += n, bcol += step) {
+                    const long long a = *G;
+                    const int a0 = (int)(a & 0x1FFFFFFF), a1 = (int)(a >> 29);
+                    const int4 b = *bcol;
+                    fx_mac(sx, a0, a1, b.x, b.y);
+                    fx_mac(sy, a0, a1, b.z, b.w);
+                }
+                const int e2 = __ldg(&ops.PinvE[(size_t)(q0 + cq) * nz + (par ? he : 0) + k]) + f - 112;
+                x = make_double2(fx_row_value(sx, e2), fx_row_value(sy, e2));
             }
-            const int e2 = __ldg(&ops.PinvE[q * nz + r]) + f - 112;
-            x = make_double2(fx_row_value(sx, e2), fx_row_value(sy, e2));
         }
-        su[r * tc + c] = x;  // su's column c was last read by the fold, before the barrier
-    }
-    __syncthreads();
-    // unfold: phi_k = pe_k + po_k, phi_nz-1-k = pe_k - po_k
-    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-        const int k = t / tc, c = t - k * tc;
-        const int m = m0 + c;
-        if (m >= g.nm || m == 0) continue;
-        const double2 pe = su[k * tc + c];
-        if (k < ho) {
-            const double2 po = su[(he + k) * tc + c];
-            PHI[(size_t)k * g.nm + m] = make_double2(pe.x + po.x, pe.y + po.y);
-            PHI[(size_t)(nz - 1 - k) * g.nm + m] = make_double2(pe.x - po.x, pe.y - po.y);
-        } else {
-            PHI[(size_t)k * g.nm + m] = pe;
-        }
+        x = pair_level(x, par);  // phi_k = pe_k + po_k | phi_nz-1-k = pe_k - po_k
+        if (!live) continue;
+        const int z = par ? nz - 1 - k : k;
+        if (m == 0) x = inv_dot(ops.PpinT + z, bpin, nz, 1);
+        PHI[(size_t)z * g.nm + m] = x;
     }
 }
 
-__global__ void __launch_bounds__(512) k_pressure_solve(GridDev g, Ops ops, double2* __restrict__ PHI) {
+__global__ void __launch_bounds__(kFxSolveThreads, 4) k_pressure_solve(GridDev g, Ops ops, double2* __restrict__ PHI) {
     pressure_solve_body(g, ops, PHI, blockIdx.x);
 }
 
@@ -3833,8 +3824,8 @@ cudaError_t launch_pressure_tc(const GridDev& g, const Ops& ops, const StepParam
     const PresRhsTcOp op{sp, US, VS, WS, PHI};
     cudaError_t e = launch_dz_tc(g, ops, op, err, s);
     if (e) return e;
-    const int tc = fx_solve_modes(g.nz);
-    k_pressure_solve<<<(g.nm + tc - 1) / tc, fx_solve_threads(g.nz), fx_solve_smem(g.nz), s>>>(g, ops, PHI);
+    const int tq = fx_solve_ops(g.nz);
+    k_pressure_solve<<<(ops.nq + tq - 1) / tq, fx_solve_threads(g.nz), fx_solve_smem(g.nz), s>>>(g, ops, PHI);
     return cudaGetLastError();
 }
 
@@ -4271,7 +4262,7 @@ int ragged_blocks(int stage, bool mixed, const RunDesc& d) {
             if (!mixed && (ragged_variant(d) & kRvViscTc)) return (d.ops.nq + d.gx[kRsVisc] - 1) / d.gx[kRsVisc];
             return tiles;
         case kRsPres:
-            if (!mixed && (ragged_variant(d) & kRvPresTc)) return (g.nm + fx_solve_modes(g.nz) - 1) / fx_solve_modes(g.nz);
+            if (!mixed && (ragged_variant(d) & kRvPresTc)) return (d.ops.nq + fx_solve_ops(g.nz) - 1) / fx_solve_ops(g.nz);
             return tiles;
         case kRsPresRhs:
             if (!mixed && (ragged_variant(d) & kRvPresTc))
