@@ -46,15 +46,29 @@ __device__ __forceinline__ unsigned fx_key(fx2 x, int e) {
 // Columns per CTA and padded transform stride (16-byte slots: one padding slot
 // after every 8, so that the passes' stores at stride 8 fall in distinct banks).
 template <int N> __host__ __device__ constexpr int yfx_ld() { return N + N / 8 + 1 - ((N + N / 8) & 1); }
-template <int N> __host__ __device__ constexpr int yfx_elems() { return per_cta(N) * yfx_ld<N>(); }
+template <int N, int CX = per_cta(N)> __host__ __device__ constexpr int yfx_elems() { return CX * yfx_ld<N>(); }
+// Columns per CTA where per_cta(N) of them leave SMs without a CTA: a quarter,
+// or half, as long as rows split evenly over the threads and a row of the tile
+// is 128 bytes.
+__host__ __device__ constexpr int per_cta_small(int n) {
+    for (int c = per_cta(n) / 4; c < per_cta(n); c *= 2)
+        if (c >= 8 && n % (kThreads / c) == 0) return c;
+    return per_cta(n);
+}
+
+// CTAs per SM the register limit leaves room for: at 4 (64 registers) the long
+// passes hide their loads better (512x384x129: the three passes 1914 -> 1820 us,
+// 96x192x81 126 -> 120), the short ones lose more to the tighter limit
+// (64x48x40 33.5 -> 38).
+__host__ __device__ constexpr int y_min_ctas(int n) { return n > 128 ? 4 : 3; }
 
 // Inverse y pass, FP64 spectra to integers: dst[f] holds X, ecol[column] its
 // exponent (column = plane * nxhp + kx).
-template <int N>
+template <int N, int CX = per_cta(N)>
 __device__ __forceinline__ void y_inv_body(const double2* __restrict__ s, fx2* __restrict__ d, int* __restrict__ ecol,
                                            const GridDev& g, int nplanes, const fx2* __restrict__ tw, int bx,
                                            fx2* buf, unsigned* emax) {
-    constexpr int CX = per_cta(N), LD = yfx_ld<N>(), B = fx_bits(N, 0);
+    constexpr int LD = yfx_ld<N>(), B = fx_bits(N, 0);
     const long long ncols = (long long)nplanes * g.nxhp;
     const int c = threadIdx.x % CX, y0 = threadIdx.x / CX;
     const long long vc = (long long)bx * CX + c;
@@ -98,11 +112,11 @@ __device__ __forceinline__ void y_inv_body(const double2* __restrict__ s, fx2* _
 // Forward y pass in place, integers (row exponents erow[plane * ny + y]) to
 // FP64 spectra, columns kx < ncol, times nl.m 2^(nl.e) = 1/(nx ny)^2 (the two
 // factors of a product of inverse transforms).
-template <int N>
+template <int N, int CX = per_cta(N)>
 __device__ __forceinline__ void y_fwd_body(fx2* __restrict__ sd, const int* __restrict__ erow, const GridDev& g,
                                            int nplanes, int ncol, const NlScale& nl, const fx2* __restrict__ tw,
                                            int bx, fx2* buf, unsigned* emax) {
-    constexpr int CX = per_cta(N), LD = yfx_ld<N>(), B = fx_bits(N, 0);
+    constexpr int LD = yfx_ld<N>(), B = fx_bits(N, 0);
     const long long ncols = (long long)nplanes * ncol;
     const int c = threadIdx.x % CX, y0 = threadIdx.x / CX;
     const long long vc = (long long)bx * CX + c;
@@ -152,21 +166,21 @@ __device__ __forceinline__ void y_fwd_body(fx2* __restrict__ sd, const int* __re
     }
 }
 
-template <int N>
-__global__ void __launch_bounds__(kThreads, 3) k_nl_y_inv(Fields src, Fields dst, int* ecol, GridDev g, int nplanes,
+template <int N, int CX>
+__global__ void __launch_bounds__(kThreads, y_min_ctas(N)) k_nl_y_inv(Fields src, Fields dst, int* ecol, GridDev g, int nplanes,
                                                           const fx2* __restrict__ tw) {
-    __shared__ fx2 buf[yfx_elems<N>()];
-    __shared__ unsigned emax[per_cta(N)];
-    y_inv_body<N>(field_ptr(src, blockIdx.z), reinterpret_cast<fx2*>(field_ptr(dst, blockIdx.z)),
+    __shared__ fx2 buf[yfx_elems<N, CX>()];
+    __shared__ unsigned emax[CX];
+    y_inv_body<N, CX>(field_ptr(src, blockIdx.z), reinterpret_cast<fx2*>(field_ptr(dst, blockIdx.z)),
                   ecol + (size_t)blockIdx.z * nplanes * g.nxhp, g, nplanes, tw, blockIdx.x, buf, emax);
 }
 
-template <int N>
-__global__ void __launch_bounds__(kThreads, 3) k_nl_y_fwd(Fields srcdst, const int* erow, GridDev g, int nplanes,
+template <int N, int CX>
+__global__ void __launch_bounds__(kThreads, y_min_ctas(N)) k_nl_y_fwd(Fields srcdst, const int* erow, GridDev g, int nplanes,
                                                           int ncol, NlScale nl, const fx2* __restrict__ tw) {
-    __shared__ fx2 buf[yfx_elems<N>()];
-    __shared__ unsigned emax[per_cta(N)];
-    y_fwd_body<N>(reinterpret_cast<fx2*>(field_ptr(srcdst, blockIdx.z)), erow + (size_t)blockIdx.z * nplanes * N, g,
+    __shared__ fx2 buf[yfx_elems<N, CX>()];
+    __shared__ unsigned emax[CX];
+    y_fwd_body<N, CX>(reinterpret_cast<fx2*>(field_ptr(srcdst, blockIdx.z)), erow + (size_t)blockIdx.z * nplanes * N, g,
                   nplanes, ncol, nl, tw, blockIdx.x, buf, emax);
 }
 
@@ -704,6 +718,17 @@ int nl_x_rows(int nxh) {
     return 1;
 }
 
+// Columns per CTA of a y pass over nf fields of ncols columns of length n.  Below
+// a CTA per SM the pass is as long as one CTA's chain (load, scale, transform,
+// store of 8 or 6 values per thread), so tiles of a quarter of the columns end
+// sooner.  us per step with full tiles and with this rule: 32x32x17 55.3 and
+// 49.1, 32x32x33 64 and 57, 64x48x40 112 and 108; with more tiles than SMs
+// there is nothing to gain.
+static int y_columns(int n, long long ncols, int nf) {
+    const int c = per_cta(n);
+    return (ncols + c - 1) / c * nf < 152 ? per_cta_small(n) : c;
+}
+
 cudaError_t nl_y_inverse(const FftCtx& ctx, const GridDev& g, Fields spec, int nf, int slot0, cudaStream_t s) {
     if (!ctx.fx || slot0 < 0 || slot0 + nf > 6) return cudaErrorInvalidValue;
     Fields tmp{};
@@ -711,11 +736,13 @@ cudaError_t nl_y_inverse(const FftCtx& ctx, const GridDev& g, Fields spec, int n
     const long long ncols = (long long)g.nz * g.nxhp;
     int* ecol = ctx.ecol + (size_t)slot0 * ncols;
     switch (g.ny) {
-#define Y_CASE(n)                                                                                      \
-    case n:                                                                                            \
-        k_nl_y_inv<n><<<dim3((unsigned)((ncols + per_cta(n) - 1) / per_cta(n)), 1, nf), kThreads, 0, s>>>( \
-            spec, tmp, ecol, g, g.nz, ctx.twq_ny);                                                     \
-        break;
+#define Y_CASE(n)                                                                          \
+    case n: {                                                                              \
+        const int cx = y_columns(n, ncols, nf);                                            \
+        auto k = cx == per_cta(n) ? k_nl_y_inv<n, per_cta(n)> : k_nl_y_inv<n, per_cta_small(n)>; \
+        k<<<dim3((unsigned)((ncols + cx - 1) / cx), 1, nf), kThreads, 0, s>>>(spec, tmp, ecol, g, g.nz, ctx.twq_ny); \
+        break;                                                                             \
+    }
         DNS3D_CT_Y_LENGTHS(Y_CASE)
 #undef Y_CASE
         default: return cudaErrorInvalidValue;
@@ -746,11 +773,15 @@ cudaError_t nl_products(const FftCtx& ctx, const GridDev& g, Fields src, int nco
     if (e) return e;
     if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_x_products");
     switch (g.ny) {
-#define Y_CASE(n)                                                                                                  \
-    case n:                                                                                                        \
-        k_nl_y_fwd<n><<<dim3((unsigned)(((long long)g.nz * ncol + per_cta(n) - 1) / per_cta(n)), 1, 3), kThreads, 0, \
-                        s>>>(src, ctx.erow, g, g.nz, ncol, ctx.nl, ctx.twq_ny);                                    \
-        break;
+#define Y_CASE(n)                                                                                              \
+    case n: {                                                                                                  \
+        const long long nc = (long long)g.nz * ncol;                                                           \
+        const int cx = y_columns(n, nc, 3);                                                                    \
+        auto k = cx == per_cta(n) ? k_nl_y_fwd<n, per_cta(n)> : k_nl_y_fwd<n, per_cta_small(n)>;                     \
+        k<<<dim3((unsigned)((nc + cx - 1) / cx), 1, 3), kThreads, 0, s>>>(src, ctx.erow, g, g.nz, ncol, ctx.nl,    \
+                                                                        ctx.twq_ny);                             \
+        break;                                                                                                 \
+    }
         DNS3D_CT_Y_LENGTHS(Y_CASE)
 #undef Y_CASE
         default: return cudaErrorInvalidValue;
