@@ -174,8 +174,10 @@ def algorithmic_bytes(wl: dict) -> dict:
     values (nq = (ny/2+1)(nx/2+1) distinct k^2, folded even/odd blocks).
       vorticity: u, v, w -> omega (6 S);
       inverse y pass: 3 fields per launch, spectrum in and out (6 S);
-      c2r x pass: 3 fields per launch (3 S + 3 R);
-      products: 6 R in, 3 R out;  r2c x pass: 3 R in, 3 S out;
+      x passes with the product: 6 S in, 3 S out; as separate kernels
+      (lengths without compile-time transforms, or on the FP64 pipe) the c2r
+      x pass: 3 fields per launch (3 S + 3 R), products: 6 R in, 3 R out, r2c
+      x pass: 3 R in, 3 S out;
       forward y pass: the kx <= kx_max columns of 3 fields, in and out;
       viscous: u, v, w, su, sv, sw in, u*, v*, w* out (9 S) + Helmholtz Inv;
       pressure: u*, v*, w* in, phi out, phi in and out (6 S) + Poisson Inv;
@@ -189,7 +191,8 @@ def algorithmic_bytes(wl: dict) -> dict:
     inv = (ny // 2 + 1) * nxhp * (he * he + ho * ho) * 8.0
     kxm = ((nx // 2) * 2) // 3 if wl.get("use_dealias_23_rule", True) else nxhp - 1
     fwd = 6 * S * min(kxm + 1, nxhp) / nxhp
-    b = {"vorticity": 6 * S, "fft_y_inverse": 6 * S, "fft_x_c2r": 3 * S + 3 * R, "products": 9 * R,
+    b = {"vorticity": 6 * S, "fft_y_inverse": 6 * S, "fft_x_products": 9 * S,
+         "fft_x_c2r": 3 * S + 3 * R, "products": 9 * R,
          "fft_x_r2c": 3 * R + 3 * S, "fft_y_forward": fwd, "viscous_helmholtz": 9 * S + inv,
          "pressure_poisson": 6 * S + inv, "pressure_correction": 9 * S, "pi_update": nz * 16.0 + 64.0}
     for k in ("vorticity", "viscous_helmholtz", "pressure_poisson", "pressure_correction"):
@@ -214,8 +217,10 @@ def working_set_note(wl: dict) -> str:
     both arms): the FP64 step re-reads its spectral state, work fields and
     per-mode inverses every step."""
     ab = algorithmic_bytes(wl)
-    # the inverse passes run as two 3-field launches per step
-    per_step = sum(v for k, v in ab.items() if not k.endswith("_tc")) + ab["fft_y_inverse"] + ab["fft_x_c2r"]
+    # the inverse y pass runs as two 3-field launches per step; the separate x
+    # kernels are not part of it
+    apart = ("fft_x_c2r", "products", "fft_x_r2c")
+    per_step = sum(v for k, v in ab.items() if not k.endswith("_tc") and k not in apart) + ab["fft_y_inverse"]
     return (f"each step moves >= {per_step / 1e6:.0f} MB of state, work fields and per-mode inverses "
             + ("> 129 MB L2, re-read every step; no flush" if per_step > 2 * 129e6
                else "(L2-resident timing; no flush)"))

@@ -3016,9 +3016,18 @@ __device__ __forceinline__ void pressure_mixed_back(const GridDev& g, const Mixe
     }
 }
 
+// Bytes of pressure_mixed_body's shared memory before the refinement's FP64
+// right-hand side.
+__host__ __device__ inline size_t pressure_mixed_base(int nz, int tc) {
+    const int ho = nz / 2, he = nz - ho, rows = (he + 3) / 4 * 4 + (ho + 3) / 4 * 4;
+    return ((size_t)(nz + 1) * tc * sizeof(float4) + 2 * (size_t)rows * tc * sizeof(float2) + 2 * (size_t)tc * sizeof(float) +
+            15) / 16 * 16;
+}
+
 // Pressure for the mixed form.  The right-hand side (the collocation
-// divergence of u*, or the weak form) is formed in FP64: D applied to the
-// full FP64 w* must not see FP32 rounding of w* (|D| ~ nz^2 would amplify it).
+// divergence of u*, or the weak form) is formed in double-float, in the weak and
+// the refined form with its terms combined in FP64: D applied to the full FP64 w*
+// must not see FP32 rounding of w* (|D| ~ nz^2 would amplify it).
 // The Neumann Poisson operator is diagonal in the eigenbasis of the full
 // problem, S V' = M V' Lambda', V'^T M V' = I:
 //   phi = -V' diag(1/(l'_j + k^2)) V'^T b,   dphi/dz = -(D V') diag(...) V'^T b
@@ -3032,14 +3041,6 @@ __device__ __forceinline__ void pressure_mixed_back(const GridDev& g, const Mixe
 // stored phi with S applied in double-float (about 2^-48 relative, against
 // the 2^-24 of the FP32 solve), and the FP32 solve of P d = r is added to
 // phi and dphi/dz: the Galerkin residual drops from ~1e-7 to ~1e-13 of b.
-// Bytes of pressure_mixed_body's shared memory before the refinement's FP64
-// right-hand side.
-__host__ __device__ inline size_t pressure_mixed_base(int nz, int tc) {
-    const int ho = nz / 2, he = nz - ho, rows = (he + 3) / 4 * 4 + (ho + 3) / 4 * 4;
-    return ((size_t)(nz + 1) * tc * sizeof(float4) + 2 * (size_t)rows * tc * sizeof(float2) + 2 * (size_t)tc * sizeof(float) +
-            15) / 16 * 16;
-}
-
 template <bool kRefine>
 __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops ops, StepParams sp,
                                                     const double2* __restrict__ US,
