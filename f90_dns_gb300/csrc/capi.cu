@@ -1161,23 +1161,6 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
             return r;
         };
         const std::vector<float2> D1e_df = split(D1e), D1o_df = split(D1o), W1e_df = split(W1e), W1o_df = split(W1o);
-        // df_dot's bounds (dns3d_internal.cuh): weights 1 / (1 - z^2) of the
-        // levels as powers of two, and the folded D1's row sums with them
-        std::vector<float> D1q(nz - nz / 2);
-        for (int j = 0; j < nz - nz / 2; ++j) {
-            const double z = h->zpts[std::max(j, 1)];
-            D1q[j] = (float)std::exp2(std::floor(-std::log2(std::max(1.0 - z * z, 1e-12))));
-        }
-        auto row_bounds = [&D1q](const std::vector<double>& a, int rows, int cols) {
-            std::vector<float> r(std::max(rows, 1), 0.f);
-            for (int i = 0; i < rows; ++i) {
-                double t = 0.0;
-                for (int j = 0; j < cols; ++j) t += std::fabs(a[(size_t)i * cols + j]) / D1q[j];
-                r[i] = t > 0.0 ? (float)std::exp2(std::ceil(std::log2(t))) : 0.f;
-            }
-            return r;
-        };
-        const std::vector<float> D1eC = row_bounds(D1e, nz - nz / 2, nz / 2), D1oC = row_bounds(D1o, nz / 2, nz - nz / 2);
         std::vector<double> Sfe, Sfo;
         fold_symmetric(S, nz, Sfe, Sfo);
         std::vector<float2> Se_df = split(Sfe), So_df = split(Sfo);
@@ -1279,8 +1262,6 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
             (rc = dev_alloc(h, &mx.PDe, PDe.size())) || (rc = dev_alloc(h, &mx.PDo, PDo.size())) ||
             (rc = dev_alloc(h, &mx.plame, plame.size())) || (rc = dev_alloc(h, &mx.plamo, plamo.size())) ||
             (rc = dev_alloc(h, &mx.D1e_df, D1e_df.size())) || (rc = dev_alloc(h, &mx.D1o_df, D1o_df.size())) ||
-            (rc = dev_alloc(h, &mx.D1eC, D1eC.size())) || (rc = dev_alloc(h, &mx.D1oC, D1oC.size())) ||
-            (rc = dev_alloc(h, &mx.D1q, D1q.size())) ||
             (rc = dev_alloc(h, &mx.W1e_df, W1e_df.size())) || (rc = dev_alloc(h, &mx.W1o_df, W1o_df.size())) ||
             (rc = dev_alloc(h, &mx.Se_df, Se_df.size())) || (rc = dev_alloc(h, &mx.So_df, So_df.size())) ||
             (rc = dev_alloc(h, &h->PHIZ, se)))
@@ -1297,8 +1278,6 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
             {mx.PDe, PDe.data(), PDe.size() * 4}, {mx.PDo, PDo.data(), PDo.size() * 4},
             {mx.plame, plame.data(), plame.size() * 4}, {mx.plamo, plamo.data(), plamo.size() * 4},
             {mx.D1e_df, D1e_df.data(), D1e_df.size() * 8}, {mx.D1o_df, D1o_df.data(), D1o_df.size() * 8},
-            {mx.D1eC, D1eC.data(), D1eC.size() * 4}, {mx.D1oC, D1oC.data(), D1oC.size() * 4},
-            {mx.D1q, D1q.data(), D1q.size() * 4},
             {mx.W1e_df, W1e_df.data(), W1e_df.size() * 8}, {mx.W1o_df, W1o_df.data(), W1o_df.size() * 8},
             {mx.Se_df, Se_df.data(), Se_df.size() * 8}, {mx.So_df, So_df.data(), So_df.size() * 8}};
         for (auto& u : u32)

@@ -250,11 +250,6 @@ struct MixedOps {
     // (hi = (float)x, lo = (float)(x - hi)) for the divergence right-hand side
     float2* D1e_df; float2* D1o_df;
     float2* W1e_df; float2* W1o_df;
-    // df_dot's bounds: q_j, powers of two near 1 / (1 - z_j^2) (at a wall its
-    // neighbour's) [he], and powers of two at least sum_j |D1e[k][j]| / q_j
-    // [he], sum_j |D1o[k][j]| / q_j [ho]: D1's rows grow like nz^2 at the walls,
-    // where w* vanishes
-    float* D1q; float* D1eC; float* D1oC;
     int nzp;                 // nz rounded up to a multiple of 4
     // interior eigenbasis, folded: the interior problem is centro-symmetric, so
     // its eigenvectors are even or odd and the basis splits into an even block

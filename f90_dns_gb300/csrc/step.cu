@@ -2747,11 +2747,23 @@ __global__ void __launch_bounds__(256) k_viscous_mixed(GridDev g, MixedOps mx, O
 struct DF {
     float hi, lo;
 };
-__device__ __forceinline__ DF df_split(double x) {
-    DF r;
-    r.hi = d2f(x);
-    r.lo = d2f(x - f2d(r.hi));
-    return r;
+// x with integer operations alone (an FP64 subtraction takes the time of 80
+// FP32 ones here): the mantissa's top 24 bits, rounded half up, and the signed
+// rest rounded to 24.  Non-finite x gives NaN.
+__device__ __forceinline__ DF df_split_bits(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7FFu), fe = e - 896;  // biased float exponent
+    const unsigned sg = hi & 0x80000000u;
+    const unsigned rest = lo & 0x1FFFFFFFu, up = rest >> 28;
+    const unsigned m = (((hi & 0xFFFFFu) << 3) | (lo >> 29)) + up;  // without the implicit bit
+    const float r = (float)((int)rest - (int)(up << 29));  // x = (2^23 + m) 2^(e-1046) + r 2^(e-1075)
+    DF d;
+    d.hi = fe > 0 ? __uint_as_float(sg | (((unsigned)fe << 23) + m)) : __uint_as_float(sg);
+    const unsigned rb = __float_as_uint(r);
+    const int le = (int)((rb >> 23) & 0xFFu) + e - 1075;  // biased exponent of the rest
+    d.lo = (rb != 0u && le > 0) ? __uint_as_float((rb + ((unsigned)(e - 1075) << 23)) ^ sg) : 0.f;
+    if (e >= 896 + 255) d.hi = d.lo = __uint_as_float(0x7FC00000u);
+    return d;
 }
 // s += a * b, a and b double-float
 // (the _rn intrinsics are never contracted into FMAs, which would break the
@@ -2789,56 +2801,13 @@ __device__ __forceinline__ void fold_load_df(float4* tile, const double2* __rest
                 fe = a;
             }
         }
-        const DF ex = df_split(fe.x), ey = df_split(fe.y);
+        const DF ex = df_split_bits(fe.x), ey = df_split_bits(fe.y);
         tile[t] = make_float4(ex.hi, ex.lo, ey.hi, ey.lo);
         if (k < ho) {
-            const DF ox = df_split(fo.x), oy = df_split(fo.y);
+            const DF ox = df_split_bits(fo.x), oy = df_split_bits(fo.y);
             tile[(he + k) * tc + c] = make_float4(ox.hi, ox.lo, oy.hi, oy.lo);
         }
     }
-}
-
-// df_split with integer operations alone (an FP64 subtraction takes the time
-// of 80 FP32 ones here): the mantissa's top 24 bits, rounded half up, and the
-// signed rest.  Non-finite x gives NaN.
-__device__ __forceinline__ DF df_split_bits(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const int e = (int)((hi >> 20) & 0x7FFu), fe = e - 896;  // biased float exponent
-    const unsigned sg = hi & 0x80000000u;
-    const unsigned rest = lo & 0x1FFFFFFFu, up = rest >> 28;
-    const unsigned m = (((hi & 0xFFFFFu) << 3) | (lo >> 29)) + up;  // without the implicit bit
-    const float r = (float)((int)rest - (int)(up << 29));  // x = (2^23 + m) 2^(e-1046) + r 2^(e-1075)
-    DF d;
-    d.hi = fe > 0 ? __uint_as_float(sg | (((unsigned)fe << 23) + m)) : __uint_as_float(sg);
-    const unsigned rb = __float_as_uint(r);
-    const int le = (int)((rb >> 23) & 0xFFu) + e - 1075;  // biased exponent of the rest
-    d.lo = (rb != 0u && le > 0) ? __uint_as_float((rb + ((unsigned)(e - 1075) << 23)) ^ sg) : 0.f;
-    if (e >= 896 + 255) d.hi = d.lo = __uint_as_float(0x7FC00000u);
-    return d;
-}
-__device__ __forceinline__ DF df_neg(DF a) { return {-a.hi, -a.lo}; }
-// a + b (Knuth's two-sum of the high parts)
-__device__ __forceinline__ DF df_add(DF a, DF b) {
-    const float t = __fadd_rn(a.hi, b.hi), z = __fsub_rn(t, a.hi);
-    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(t, z)), __fsub_rn(b.hi, z));
-    return {t, __fadd_rn(__fadd_rn(a.lo, b.lo), e)};
-}
-__device__ __forceinline__ void df_mac(DF& s, DF a, DF b) { df_mac(s, a.hi, a.lo, b.hi, b.lo); }
-
-// Dot products of double-floats with a bound known beforehand: the high sum
-// starts at c = 3 2^q with 2^q >= sum |a_i b_i|, so it stays in [2^(q+1), 2^(q+2)]
-// and is always the larger addend: t = fma(a, b, s) and t - s are then exact but
-// for t's rounding, which fma(a, b, s - t) recovers -- 6 FP32 instructions per
-// term against the 12 of df_mac.  Errors are 2^-46 of the bound: for D1.w* of
-// evolved channel fields at most 1.2e-11 (nz = 33) to 3.5e-10 (nz = 193) of the
-// column's largest right-hand side, whose rounding to FP32 after it is 6e-8.
-__device__ __forceinline__ void df_dot(DF& s, float ahi, float alo, float bhi, float blo) {
-    const float t = fmaf(ahi, bhi, s.hi);
-    const float z = __fsub_rn(s.hi, t);
-    s.lo = __fadd_rn(s.lo, fmaf(ahi, bhi, z));
-    s.lo = fmaf(ahi, blo, s.lo);
-    s.lo = fmaf(alo, bhi, s.lo);
-    s.hi = t;
 }
 
 // anti_apply_df's even and odd parts before their sum and difference:
@@ -3020,14 +2989,12 @@ __device__ __forceinline__ void pressure_mixed_back(const GridDev& g, const Mixe
 // right-hand side.
 __host__ __device__ inline size_t pressure_mixed_base(int nz, int tc) {
     const int ho = nz / 2, he = nz - ho, rows = (he + 3) / 4 * 4 + (ho + 3) / 4 * 4;
-    return ((size_t)(nz + 1) * tc * sizeof(float4) + 2 * (size_t)rows * tc * sizeof(float2) + 2 * (size_t)tc * sizeof(float) +
-            15) / 16 * 16;
+    return ((size_t)nz * tc * sizeof(float4) + 2 * (size_t)rows * tc * sizeof(float2) + (size_t)tc * sizeof(float) + 15) / 16 * 16;
 }
 
 // Pressure for the mixed form.  The right-hand side (the collocation
-// divergence of u*, or the weak form) is formed in double-float, in the weak and
-// the refined form with its terms combined in FP64: D applied to the full FP64 w*
-// must not see FP32 rounding of w* (|D| ~ nz^2 would amplify it).
+// divergence of u*, or the weak form) is formed in FP64: D applied to the
+// full FP64 w* must not see FP32 rounding of w* (|D| ~ nz^2 would amplify it).
 // The Neumann Poisson operator is diagonal in the eigenbasis of the full
 // problem, S V' = M V' Lambda', V'^T M V' = I:
 //   phi = -V' diag(1/(l'_j + k^2)) V'^T b,   dphi/dz = -(D V') diag(...) V'^T b
@@ -3052,141 +3019,62 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
     const int nz = g.nz, he = ops.he, ho = ops.ho;
     const int pe4 = mx.phe4, po4 = mx.pho4;
     float4* tw = reinterpret_cast<float4*>(smraw);              // folded w* (double-float)  [nz][tc]
-    float4* ta = tw + nz * tc;                                  // (i ax / 2, i ay / 2) as double-floats [tc]
-    float2* tb = reinterpret_cast<float2*>(ta + tc);            // folded rhs: s [pe4][tc], d [po4][tc]
+    float2* tb = reinterpret_cast<float2*>(tw + nz * tc);       // folded rhs: s [pe4][tc], d [po4][tc]
     float2* tp = tb + (pe4 + po4) * tc;                         // phi~: even [pe4][tc], odd [po4][tc]
     float* tk = reinterpret_cast<float*>(tp + (pe4 + po4) * tc);  // k^2 [tc]
-    unsigned* tm = reinterpret_cast<unsigned*>(tk + tc);        // largest q |re|, q |im| of the folded column (float bits)
     double2* bt = reinterpret_cast<double2*>(smraw + pressure_mixed_base(nz, tc));  // FP64 rhs [nz][tc] (refinement)
     const int m0 = bx * tc;
     const bool strong = !kRefine && !sp.weak_form;
     const TileDiv td = tile_div(tc);
     for (int c = threadIdx.x; c < tc; c += blockDim.x) {
         const int m = min(m0 + c, g.nm - 1);
-        const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
-        const DF ax = df_split_bits(0.5 * mi.ax), ay = df_split_bits(0.5 * mi.ay);
-        ta[c] = make_float4(ax.hi, ax.lo, ay.hi, ay.lo);
-        tk[c] = d2f(__ldg(&ops.ksq[mode_q(mi.ky, mi.kx, g.ny, g.nxhp)]));
-        tm[c] = 0u;
+        const int ky = m / g.nxhp, kx = m - ky * g.nxhp;
+        tk[c] = d2f(__ldg(&ops.ksq[mode_q(ky, kx, g.ny, g.nxhp)]));
     }
+    fold_load_df(tw, WS, g, m0, tc, he, ho);
     for (int t = threadIdx.x; t < (pe4 - he) * tc; t += blockDim.x) tb[he * tc + t] = make_float2(0.f, 0.f);
     for (int t = threadIdx.x; t < (po4 - ho) * tc; t += blockDim.x) tb[(pe4 + ho) * tc + t] = make_float2(0.f, 0.f);
-    if (strong) {
-        __syncthreads();  // tm zeroed
-        // w* as double-floats, folded, and each column's largest component
-        // weighted by q (MixedOps)
-        for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-            const int k = tile_row(td, t), c = t - k * tc;
-            const int m = m0 + c;
-            float4 fe = make_float4(0.f, 0.f, 0.f, 0.f), fo = fe;
-            if (m < g.nm) {
-                const double2 a = WS[(size_t)k * g.nm + m];
-                const DF ax = df_split_bits(a.x), ay = df_split_bits(a.y);
-                fe = make_float4(ax.hi, ax.lo, ay.hi, ay.lo);
+    __syncthreads();
+    const float2* __restrict__ Ae = sp.weak_form ? mx.W1e_df : mx.D1e_df;
+    const float2* __restrict__ Ao = sp.weak_form ? mx.W1o_df : mx.D1o_df;
+    // right-hand side pair (k, nz-1-k), folded in FP64 before the rounding
+    for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
+        const int k = tile_row(td, t), c = t - k * tc;
+        const int m = m0 + c;
+        float2 fs = make_float2(0.f, 0.f), fd = fs;
+        double2 b1 = make_double2(0.0, 0.0), b2 = b1;
+        if (m < g.nm && m != 0) {
+            const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
+            if (strong) {
+                // the folded strong-form right-hand side divided by 2 w_k / dt
+                // (the scaled forward operators PAeS, PAoS carry that factor):
+                // (b_k +- b_k') dt / (2 w_k) = i (ax/2)(u_k +- u_k') +
+                // i (ay/2)(v_k +- v_k') + (ye | yo), the mid level
+                // i (ax/2) u_k + i (ay/2) v_k + ye / 2; ye, yo the even and
+                // odd parts of D1.w* -- 20 FP64 operations per level pair
+                // instead of 36.  They stay in FP64 and D1.w* in double-float
+                // with its own rounding errors only: the divergence of u* is
+                // dt times a source, so the terms cancel.  In double-float,
+                // with the sums held against a bound, the kernel took 49
+                // instead of 57 us (128x128x65) and 325 instead of 354
+                // (256x256x97), and the projection's residual at dt = 1e-8
+                // went from 4e-6 to 5e-5 (nz = 33), 3e-5 to 2e-4 (65)
+                const double4 y = anti_apply_df_parts(Ae, Ao, tw, k, c, tc, he, ho);
+                const double hax = 0.5 * mi.ax, hay = 0.5 * mi.ay;
+                const size_t o1 = (size_t)k * g.nm + m;
+                const double2 u1 = US[o1], v1 = VS[o1];
                 if (k < ho) {
-                    const double2 b = WS[(size_t)(nz - 1 - k) * g.nm + m];
-                    const DF bx_ = df_split_bits(b.x), by = df_split_bits(b.y);
-                    const DF px = df_add(ax, bx_), py = df_add(ay, by);
-                    const DF mx_ = df_add(ax, df_neg(bx_)), my = df_add(ay, df_neg(by));
-                    fe = make_float4(px.hi, px.lo, py.hi, py.lo);
-                    fo = make_float4(mx_.hi, mx_.lo, my.hi, my.lo);
-                }
-            }
-            tw[t] = fe;
-            if (k < ho) tw[(he + k) * tc + c] = fo;
-            const unsigned mag = 0x7FFFFFFFu;
-            const unsigned big = max(max(__float_as_uint(fe.x) & mag, __float_as_uint(fe.z) & mag),
-                                     max(__float_as_uint(fo.x) & mag, __float_as_uint(fo.z) & mag));
-            atomicMax(&tm[c], __float_as_uint(__uint_as_float(big) * __ldg(&mx.D1q[k])));
-        }
-        __syncthreads();
-        // The folded strong-form right-hand side divided by 2 w_k / dt (the
-        // scaled forward operators PAeS, PAoS carry that factor), all in
-        // double-float: (b_k +- b_k') dt / (2 w_k) = i (ax/2)(u_k +- u_k') +
-        // i (ay/2)(v_k +- v_k') + (ye | yo), the mid level i (ax/2) u_k +
-        // i (ay/2) v_k + ye / 2; ye, yo the even and odd parts of D1.w*.
-        // With the combination in FP64 (20 operations per level pair, each the
-        // time of 80 FP32 ones) the kernel took 63 us at 128x128x65, 354 us at
-        // 256x256x97; now 48 and 307.
-        for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-            const int k = tile_row(td, t), c = t - k * tc;
-            const int m = m0 + c;
-            float2 fs = make_float2(0.f, 0.f), fd = fs;
-            if (m < g.nm && m != 0) {
-                const size_t o1 = (size_t)k * g.nm + m, o2 = (size_t)(nz - 1 - k) * g.nm + m;
-                const double2 u1 = US[o1], v1 = VS[o1], u2 = US[o2], v2 = VS[o2];
-                // the column's largest weighted component as a power of two above it
-                const float cm = __uint_as_float((tm[c] & 0x7F800000u) + 0x00800000u);
-                const float ce = 3.f * cm * __ldg(&mx.D1eC[k]);
-                DF yex{ce, 0.f}, yey{ce, 0.f}, yox{0.f, 0.f}, yoy{0.f, 0.f};
-                {
-                    const float2* er = mx.D1e_df + (size_t)k * ho;
-                    const float4* f = tw + he * tc + c;
-#pragma unroll 4
-                    for (int j = 0; j < ho; ++j) {
-                        const float2 a = __ldg(&er[j]);
-                        const float4 b = f[j * tc];
-                        df_dot(yex, a.x, a.y, b.x, b.y);
-                        df_dot(yey, a.x, a.y, b.z, b.w);
-                    }
-                    yex.hi -= ce;
-                    yey.hi -= ce;
-                }
-                const float4 ma = ta[c];
-                const DF hax{ma.x, ma.y}, hay{ma.z, ma.w}, nax = df_neg(hax), nay = df_neg(hay);
-                const DF u1x = df_split_bits(u1.x), u1y = df_split_bits(u1.y);
-                const DF v1x = df_split_bits(v1.x), v1y = df_split_bits(v1.y);
-                if (k < ho) {
-                    const float co = 3.f * cm * __ldg(&mx.D1oC[k]);
-                    yox.hi = yoy.hi = co;
-                    const float2* orow = mx.D1o_df + (size_t)k * he;
-                    const float4* f = tw + c;
-#pragma unroll 4
-                    for (int j = 0; j < he; ++j) {
-                        const float2 a = __ldg(&orow[j]);
-                        const float4 b = f[j * tc];
-                        df_dot(yox, a.x, a.y, b.x, b.y);
-                        df_dot(yoy, a.x, a.y, b.z, b.w);
-                    }
-                    yox.hi -= co;
-                    yoy.hi -= co;
-                    const DF u2x = df_split_bits(u2.x), u2y = df_split_bits(u2.y);
-                    const DF v2x = df_split_bits(v2.x), v2y = df_split_bits(v2.y);
-                    df_mac(yex, nax, df_add(u1y, u2y));
-                    df_mac(yex, nay, df_add(v1y, v2y));
-                    df_mac(yey, hax, df_add(u1x, u2x));
-                    df_mac(yey, hay, df_add(v1x, v2x));
-                    df_mac(yox, nax, df_add(u1y, df_neg(u2y)));
-                    df_mac(yox, nay, df_add(v1y, df_neg(v2y)));
-                    df_mac(yoy, hax, df_add(u1x, df_neg(u2x)));
-                    df_mac(yoy, hay, df_add(v1x, df_neg(v2x)));
-                    fd = make_float2(yox.hi + yox.lo, yoy.hi + yoy.lo);
+                    const size_t o2 = (size_t)(nz - 1 - k) * g.nm + m;
+                    const double2 u2 = US[o2], v2 = VS[o2];
+                    const double2 up = make_double2(u1.x + u2.x, u1.y + u2.y), um = make_double2(u1.x - u2.x, u1.y - u2.y);
+                    const double2 vp = make_double2(v1.x + v2.x, v1.y + v2.y), vm = make_double2(v1.x - v2.x, v1.y - v2.y);
+                    fs = make_float2(d2f(fma(-hax, up.y, fma(-hay, vp.y, y.x))), d2f(fma(hax, up.x, fma(hay, vp.x, y.y))));
+                    fd = make_float2(d2f(fma(-hax, um.y, fma(-hay, vm.y, y.z))), d2f(fma(hax, um.x, fma(hay, vm.x, y.w))));
                 } else {
-                    yex = DF{0.5f * yex.hi, 0.5f * yex.lo};
-                    yey = DF{0.5f * yey.hi, 0.5f * yey.lo};
-                    df_mac(yex, nax, u1y);
-                    df_mac(yex, nay, v1y);
-                    df_mac(yey, hax, u1x);
-                    df_mac(yey, hay, v1x);
+                    fs = make_float2(d2f(fma(-hax, u1.y, fma(-hay, v1.y, 0.5 * y.x))),
+                                     d2f(fma(hax, u1.x, fma(hay, v1.x, 0.5 * y.y))));
                 }
-                fs = make_float2(yex.hi + yex.lo, yey.hi + yey.lo);
-            }
-            tb[k * tc + c] = fs;
-            if (k < ho) tb[(pe4 + k) * tc + c] = fd;
-        }
-    } else {
-        fold_load_df(tw, WS, g, m0, tc, he, ho);
-        __syncthreads();
-        const float2* __restrict__ Ae = sp.weak_form ? mx.W1e_df : mx.D1e_df;
-        const float2* __restrict__ Ao = sp.weak_form ? mx.W1o_df : mx.D1o_df;
-        // right-hand side pair (k, nz-1-k), folded in FP64 before the rounding
-        for (int t = threadIdx.x; t < he * tc; t += blockDim.x) {
-            const int k = tile_row(td, t), c = t - k * tc;
-            const int m = m0 + c;
-            float2 fs = make_float2(0.f, 0.f), fd = fs;
-            double2 b1 = make_double2(0.0, 0.0), b2 = b1;
-            if (m < g.nm && m != 0) {
-                const ModeInfo mi = mode_info(g, m, ops.xw, ops.yw);
+            } else {
                 const Pair dz = anti_apply_df(Ae, Ao, tw, k, c, tc, he, ho);
                 b1 = pressure_rhs(g, ops, sp, k, m, mi, US, VS, dz.a);
                 if (k < ho) {
@@ -3197,12 +3085,12 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
                     fs = make_float2(d2f(b1.x), d2f(b1.y));
                 }
             }
-            tb[k * tc + c] = fs;
-            if (k < ho) tb[(pe4 + k) * tc + c] = fd;
-            if (kRefine) {
-                bt[k * tc + c] = b1;
-                if (k < ho) bt[(nz - 1 - k) * tc + c] = b2;
-            }
+        }
+        tb[k * tc + c] = fs;
+        if (k < ho) tb[(pe4 + k) * tc + c] = fd;
+        if (kRefine) {
+            bt[k * tc + c] = b1;
+            if (k < ho) bt[(nz - 1 - k) * tc + c] = b2;
         }
     }
     __syncthreads();
@@ -3858,9 +3746,10 @@ cudaError_t launch_pressure_mixed(const GridDev& g, const MixedOps& mx, const Op
                                   double2* PHIZ, cudaStream_t s) {
     const int tc = tile_width(g, kTilePresM);
     const size_t sm = pressure_mixed_smem(g, tc);
-    // 16 warps hide the latency of the matrix rows (us, 256 -> 512 threads:
-    // 128x128x65 51.4 -> 48.3, 192x96x58 refined 110.8 -> 110.6, 256x256x97
-    // 324 -> 307, 64x48x40 18.4 either way)
+    // 16 warps for the latency of the matrix rows, which the right-hand side's
+    // FP64 operations leave little of (us, 256 and 512 threads: 96x96x49 28.7 and
+    // 26.6, 128x128x65 57.3 and 57.4, 256x256x97 353 and 354, 192x96x58 refined
+    // 100 and 104)
     const int nt = 512;
     if (sp.refine)
         k_pressure_mixed<true><<<(g.nm + tc - 1) / tc, nt, sm, s>>>(g, mx, ops, sp, US, VS, WS, PHI, PHIZ, tc);
