@@ -292,9 +292,11 @@ __device__ __forceinline__ void c2r_x_body_fx(const Fields& src, const RFields& 
     }
     __syncthreads();
     ct_fft<N, 1, +1, RX, LD>(buf, tw_n);
-    // 1/(nx ny) = M 2^(E - 1075), M its 53-bit mantissa: Y = round(Z (M 2^9) / 2^63)
+    // 1/(nx ny) = M 2^(E - 1075), M its 53-bit mantissa: Y = round(Z M / 2^52),
+    // no coarser than Z (over 2^63, as the limb products give it, a constant
+    // field came back two bits short)
     const long long sb = __double_as_longlong(g.inv_nxny);
-    const FxLimbs M = fx_split<9>((sb & 0xFFFFFFFFFFFFFLL) | (1LL << 52));
+    const long long M = (sb & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
     const int E = (int)((sb >> 52) & 0x7FF);
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
@@ -302,9 +304,10 @@ __device__ __forceinline__ void c2r_x_body_fx(const Fields& src, const RFields& 
         const int r = t / N, k = t - r * N;
         if (row0 + r < nrows) {
             const int em = (int)emax[r];
-            const int e2 = em + E - 2043 - B;
+            const int e2 = em + E - 2045 - B;
             const fx2 z = buf[r * LD + sw<fx2>(k)];
-            const long long yx = fx_mulq(z.x, M), yy = fx_mulq(z.y, M);
+            const long long yx = (long long)(((__int128)z.x * M + ((__int128)1 << 51)) >> 52);
+            const long long yy = (long long)(((__int128)z.y * M + ((__int128)1 << 51)) >> 52);
             const double2 o =
                 em == 0x7FF ? make_double2(fx_nan(), fx_nan()) : make_double2(fx_to(yx, e2), fx_to(yy, e2));
             d[(size_t)(row0 + r) * N + k] = o;
