@@ -107,8 +107,18 @@ int cuda_fail(dns3d_handle* h, cudaError_t e, const char* what) {
 size_t spec_elems(const dns3d_config& c) { return (size_t)(c.nx / 2 + 1) * c.ny * c.nz; }
 size_t phys_elems(const dns3d_config& c) { return (size_t)c.nx * c.ny * c.nz; }
 int n_unique_q(const dns3d_config& c) { return (c.ny / 2 + 1) * (c.nx / 2 + 1); }
-// k^2 values whose Helmholtz and Poisson inverses a handle builds
-int n_inverses(const dns3d_config& c) { return c.precision == DNS3D_PREC_MIXED ? 2 : n_unique_q(c); }
+// k^2 values whose Helmholtz and Poisson inverses a handle builds.  The mixed form
+// solves every mode but (0,0) in the eigenbases: it builds that mode's and, for
+// the refusal of a k^2 that overflows, the largest k^2's (96x96x65: 2.2 ms and
+// 110 MB less than all).  A small k^2 can be refused too: where k^2 M is lost
+// beside S, the Poisson operator is S alone and its last pivot may be zero (it
+// is at nz = 3 from xlen = 1e9 on).  Boxes with a k^2 below 2^-33 (6e5 long),
+// 2^20 above the rounding of entries near 1, build them all.
+int n_inverses(const dns3d_config& c) {
+    const double kx = 2.0 * kPi / c.xlen, ky = 2.0 * kPi / c.ylen;
+    const bool shortest = std::min(kx * kx, ky * ky) >= 0x1.0p-33;
+    return c.precision == DNS3D_PREC_MIXED && shortest ? 2 : n_unique_q(c);
+}
 
 size_t footprint(const dns3d_config& c);
 constexpr size_t kTableBytes = 16ull << 20;  // footprint's allowance for operators, tables, reductions
@@ -1018,10 +1028,7 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     ops.he = nz - ops.ho;
     const size_t nz2 = (size_t)nz * nz;
     const size_t qstride = (size_t)ops.he * ops.he + (size_t)ops.ho * ops.ho;
-    // The mixed form solves every mode but (0,0) in the eigenbases: it builds that
-    // mode's inverses and, for the refusal of a k^2 that overflows, the largest
-    // k^2's.  A 96x96x65 handle: 2.2 ms and 110 MB for all of them.
-    const int nqi = n_inverses(c);
+    const int nqi = n_inverses(c);  // q = 0 and the largest k^2, or all of them
     const double ksq_ends[2] = {ksq.front(), ksq.back()};
     double* d_ksq = nullptr;
     double* dS = nullptr;

@@ -207,7 +207,7 @@ struct Ops {
     double* yw;      // [ny]
     double* ksq;     // xsq+ysq per unique q     [nq]
     double* S;       // stiffness (2/ybar) sum_m d1(m,k) d1(m,n) zwts(m), [nz][nz] (jacgs)
-    double* HinvF;   // folded Helmholtz inverses      [nq][he*he + ho*ho] (mixed: q = 0 only)
+    double* HinvF;   // folded Helmholtz inverses      [nq][he*he + ho*ho] (mixed: q = 0 read)
     double* PinvF;   // folded Poisson inverses        [nq][he*he + ho*ho] (mixed: none read)
     double* PpinT;   // pinned (0,0) Poisson inverse, unfolded, transposed [nz][nz]
     // PinvF in 58-bit fixed point for the solve on the integer pipes (FP64
