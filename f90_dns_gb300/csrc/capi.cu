@@ -57,6 +57,10 @@ struct dns3d_handle {
     // viscous solve on the tensor cores (ops.tcA built): chosen by the tile
     // autotuner unless DNS3D_TENSOR_CORES forces it (1) or rules it out (0)
     bool visc_tc = false;
+    // whether creation builds the images of the tensor-core viscous solve and of
+    // the tensor-core z-derivatives
+    bool tc_visc = false;
+    bool tc_dz = false;
     bool visc_tc_forced = false;
     // the vorticity's and the projection's z-derivatives on the tensor cores
     // (ops.tcD built), chosen likewise
@@ -120,21 +124,26 @@ int n_inverses(const dns3d_config& c) {
     return c.precision == DNS3D_PREC_MIXED && shortest ? 2 : n_unique_q(c);
 }
 
-size_t footprint(const dns3d_config& c);
+// Device bytes of a handle, with the images of the tensor-core viscous solve
+// (digit slices) and of the tensor-core z-derivatives (digit D1, fixed-point
+// Poisson inverses) where it builds them.
+size_t footprint(const dns3d_config& c, bool tc_visc, bool tc_dz);
 constexpr size_t kTableBytes = 16ull << 20;  // footprint's allowance for operators, tables, reductions
 
-// Device memory from one allocation of the handle's size, made by the first
-// call, and from blocks of 4 MB for what exceeds it (256-byte steps; freed with
-// the handle).  A buffer each cost a handle 1.8 ms of cudaMalloc and 0.8 ms of
-// cudaFree (96x96x65, mixed; creating it 5.6 and 3.9 ms, six handles of serving
-// grids freed in 5.0 and 1.0 ms).  Every buffer starts zeroed (work
-// buffers are read by the tile autotuner).
+// Device memory from one allocation of the handle's size (of what it builds:
+// with DNS3D_TENSOR_CORES=0 no tensor-core image, half of a 128x96x129 handle),
+// made by the first call, and from blocks of 4 MB for what exceeds it (256-byte
+// steps; freed with the handle).  A buffer each cost a handle 1.8 ms of
+// cudaMalloc and 0.8 ms of cudaFree (96x96x65, mixed; creating it 5.6 and 3.9
+// ms, six handles of serving grids freed in 5.0 and 1.0 ms).  Every buffer
+// starts zeroed (work buffers are read by the tile autotuner).
 template <typename T>
 int dev_alloc(dns3d_handle* h, T** p, size_t count) {
     constexpr size_t kBlock = 4ull << 20;
     const size_t need = (std::max<size_t>(count * sizeof(T), 1) + 255) / 256 * 256;
     if (need > h->slab_left) {
-        const size_t block = std::max(need, h->allocs.empty() ? footprint(h->cfg) - kTableBytes + kBlock : kBlock);
+        const size_t block = std::max(
+            need, h->allocs.empty() ? footprint(h->cfg, h->tc_visc, h->tc_dz) - kTableBytes + kBlock : kBlock);
         void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, block);
         if (e != cudaSuccess) return cuda_fail(h, e, "cudaMalloc");
@@ -623,7 +632,7 @@ int run_step_body(dns3d_handle* h) {
     return run_correction(h, true);
 }
 
-size_t footprint(const dns3d_config& c) {
+size_t footprint(const dns3d_config& c, bool tc_visc, bool tc_dz) {
     const size_t se = spec_elems(c), pe = phys_elems(c);
     const size_t nm = (size_t)(c.nx / 2 + 1) * c.ny;
     const size_t nq = (size_t)n_unique_q(c);
@@ -647,11 +656,13 @@ size_t footprint(const dns3d_config& c) {
     }
     if (c.precision != DNS3D_PREC_MIXED && tc_supported(c.nz)) {
         const TcGeom t = tc_geom(c.nz);
-        if (c.use_crank_nicolson && c.linear_solver == 0)  // digit slices of the Helmholtz inverses
+        if (tc_visc && c.use_crank_nicolson && c.linear_solver == 0)  // digit slices of the Helmholtz inverses
             b += nq * (tc_q_halves(t) * sizeof(__half) + (size_t)t.m8 * sizeof(int));
-        b += (size_t)kTcSlices * tc_blocks(t, true).a * sizeof(__half);  // digit image of D1
-        if (!c.use_weak_form_divergence)  // fixed-point Poisson inverses and row exponents
-            b += nq * (fx_qstride((int)ez, (int)hz) * sizeof(long long) + (size_t)c.nz * sizeof(int));
+        if (tc_dz) {
+            b += (size_t)kTcSlices * tc_blocks(t, true).a * sizeof(__half);  // digit image of D1
+            if (!c.use_weak_form_divergence)  // fixed-point Poisson inverses and row exponents
+                b += nq * (fx_qstride((int)ez, (int)hz) * sizeof(long long) + (size_t)c.nz * sizeof(int));
+        }
     }
     return b + kTableBytes;
 }
@@ -719,7 +730,7 @@ int dns3d_config_read_namelist(const char* path, dns3d_config* cfg) {
 
 int dns3d_footprint_bytes(const dns3d_config* c, unsigned long long* bytes) {
     if (!c || !bytes) return DNS3D_E_INVALID;
-    *bytes = footprint(*c);
+    *bytes = footprint(*c, true, true);
     return DNS3D_OK;
 }
 
@@ -980,6 +991,11 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     g.inv_nxny = 1.0 / ((double)c.nx * (double)c.ny);
     g.refine = (c.precision == DNS3D_PREC_MIXED && c.poisson_refinement) ? 1 : 0;
     const int nz = c.nz;
+    // FP64 runs; DNS3D_TENSOR_CORES=0 keeps the FP64-pipe kernels
+    const char* tcenv = std::getenv("DNS3D_TENSOR_CORES");
+    const bool tc_on = c.precision == DNS3D_PREC_FP64 && !(tcenv && std::strcmp(tcenv, "0") == 0);
+    h->tc_visc = tc_on && c.use_crank_nicolson && c.linear_solver == 0 && viscous_tc_fits(g);
+    h->tc_dz = tc_on && vorticity_tc_fits(g);
 
     // setup_grid_3d (3D:740-742) and setup_spectral_3d (3D:769-809)
     const double ybar = 2.0;
@@ -1327,15 +1343,13 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     pp.inv_nxny_wsum = 1.0 / ((double)c.nx * (double)c.ny * wsum);
 
     // tensor-core form of the Helmholtz inverses: FP64 Crank-Nicolson runs with
-    // the direct solver (DNS3D_TENSOR_CORES=0 keeps the FP64-pipe kernel)
+    // the direct solver
     if ((rc = dev_alloc(h, &h->d_tcerr, 2))) return fail(rc);
     const char* zcenv = std::getenv("DNS3D_ZERO_COPY");
     h->zero_copy = !(zcenv && std::strcmp(zcenv, "0") == 0);
-    const char* tcenv = std::getenv("DNS3D_TENSOR_CORES");
     const char* stall = std::getenv("DNS3D_TC_TEST_STALL");
     ops.tc_stall = stall && std::strcmp(stall, "1") == 0;
-    if (!h->mixed && sp.cn_identity && c.linear_solver == 0 && !(tcenv && std::strcmp(tcenv, "0") == 0) &&
-        viscous_tc_fits(g)) {
+    if (h->tc_visc && sp.cn_identity) {
         const TcGeom t = tc_geom(nz);
         __half* sl = nullptr;
         int* ex = nullptr;
@@ -1368,7 +1382,7 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
         h->visc_tc = h->visc_tc_forced || (nq >= 8 * 152 && viscous_tc_smem(g) <= 113 * 1024);
     }
     // the folded D1 as a digit image for the tensor-core vorticity (FP64 runs)
-    if (!h->mixed && !(tcenv && std::strcmp(tcenv, "0") == 0) && vorticity_tc_fits(g)) {
+    if (h->tc_dz) {
         const TcGeom t = tc_geom(nz);
         __half* im = nullptr;
         int* ex = nullptr;
