@@ -3079,8 +3079,11 @@ __device__ __forceinline__ void pressure_mixed_body(GridDev g, MixedOps mx, Ops 
                 b1 = pressure_rhs(g, ops, sp, k, m, mi, US, VS, dz.a);
                 if (k < ho) {
                     b2 = pressure_rhs(g, ops, sp, nz - 1 - k, m, mi, US, VS, dz.b);
-                    fs = make_float2(d2f(b1.x + b2.x), d2f(b1.y + b2.y));
-                    fd = make_float2(d2f(b1.x - b2.x), d2f(b1.y - b2.y));
+                    // (explicit roundings: where u* is solenoidal the difference is of
+                    // equal values, and a product contracted into it would leave
+                    // a residue in one instantiation and none in another)
+                    fs = make_float2(d2f(__dadd_rn(b1.x, b2.x)), d2f(__dadd_rn(b1.y, b2.y)));
+                    fd = make_float2(d2f(__dsub_rn(b1.x, b2.x)), d2f(__dsub_rn(b1.y, b2.y)));
                 } else {
                     fs = make_float2(d2f(b1.x), d2f(b1.y));
                 }
