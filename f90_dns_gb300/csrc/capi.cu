@@ -2188,7 +2188,6 @@ RunDesc make_desc(const dns3d_handle* h) {
         for (int f = 0; f < 6; ++f) {
             d.spec[f] = f < 3 ? static_cast<void*>(f == 0 ? h->U : f == 1 ? h->V : h->W) : h->spec32[f];
             d.tmp[f] = h->fft.tmp32 + (size_t)f * se;
-            d.phys[f] = h->phys32[f];
         }
         for (int f = 0; f < 3; ++f) d.src[f] = h->src32[f];
         d.tw_ny = h->fft.tw32_ny; d.tw_nx2 = h->fft.tw32_nx2; d.tw_nx = h->fft.tw32_nx;

@@ -118,12 +118,10 @@ bool fft_ct_supported(int ny, int nxh);
 template <int SIGN, typename C>
 cudaError_t fft_ct_y(FieldsT<C> src, FieldsT<C> dst, const GridDev& g, int nplanes, int ncol, int nf, const C* tw,
                      cudaStream_t s);
-template <typename T>
-cudaError_t fft_ct_c2r_x(FieldsT<typename Cx<T>::type> src, FieldsT<T> dst, const GridDev& g, int nrows, int nf,
-                         const typename Cx<T>::type* tw_n, const typename Cx<T>::type* tw_nx, cudaStream_t s);
-template <typename T>
-cudaError_t fft_ct_r2c_x(FieldsT<T> src, FieldsT<typename Cx<T>::type> dst, const GridDev& g, int nrows, int nf,
-                         const typename Cx<T>::type* tw_n, const typename Cx<T>::type* tw_nx, cudaStream_t s);
+cudaError_t fft_ct_c2r_x(Fields src, RFields dst, const GridDev& g, int nrows, int nf, const double2* tw_n,
+                         const double2* tw_nx, cudaStream_t s);
+cudaError_t fft_ct_r2c_x(RFields src, Fields dst, const GridDev& g, int nrows, int nf, const double2* tw_n,
+                         const double2* tw_nx, cudaStream_t s);
 
 // The FP64 passes of fft_ct in block fixed point (Q62 twiddle tables).
 template <int SIGN>
@@ -165,7 +163,8 @@ cudaError_t fft_c2r_copy(const FftCtx& ctx, const GridDev& g, Fields spec, RFiel
 // 2/3 filter truncates at kx_max = ncol - 1 anyway.
 cudaError_t fft_r2c(const FftCtx& ctx, const GridDev& g, RFields phys, Fields spec, int nf,
                     int nplanes, cudaStream_t s, int ncol = 0, bool host_src = false);
-// FP32 versions (same transform definitions), scratch ctx.tmp32.
+// FP32 versions (same transform definitions) for the lengths without
+// compile-time kernels (the others: nl_transforms32), scratch ctx.tmp32.
 cudaError_t fft_c2r32(const FftCtx& ctx, const GridDev& g, FFields spec, FRFields phys, int nf,
                       int nplanes, cudaStream_t s);
 cudaError_t fft_r2c32(const FftCtx& ctx, const GridDev& g, FRFields phys, FFields spec, int nf,

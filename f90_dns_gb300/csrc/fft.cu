@@ -395,14 +395,14 @@ cudaError_t c2r_impl(const FftCtx& ctx, const GridDev& g, FieldsT<typename Cx<T>
             if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_x_c2r");
             return e;
         }
-    }
-    if (ctx.use_ct) {
-        cudaError_t e = fft_ct_y<+1, C>(spec, tmp, g, nplanes, g.nxhp, nf, twy, s);
-        if (e) return e;
-        if (ctx.hook) ctx.hook(ctx.hook_ctx, sizeof(T) == 8 ? "fft_y_inverse" : "fft32_y_inverse");
-        e = fft_ct_c2r_x<T>(tmp, phys, g, nrows, nf, twx2, twx, s);
-        if (ctx.hook) ctx.hook(ctx.hook_ctx, sizeof(T) == 8 ? "fft_x_c2r" : "fft32_x_c2r");
-        return e;
+        if (ctx.use_ct) {
+            cudaError_t e = fft_ct_y<+1, C>(spec, tmp, g, nplanes, g.nxhp, nf, twy, s);
+            if (e) return e;
+            if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_y_inverse");
+            e = fft_ct_c2r_x(tmp, phys, g, nrows, nf, twx2, twx, s);
+            if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_x_c2r");
+            return e;
+        }
     }
     const int cx = pick_cx(g.ny);
     dim3 gy((g.nxhp + cx - 1) / cx, nplanes, nf);
@@ -432,14 +432,14 @@ cudaError_t r2c_impl(const FftCtx& ctx, const GridDev& g, FieldsT<T> phys, Field
             if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_y_forward");
             return e;
         }
-    }
-    if (ctx.use_ct) {
-        cudaError_t e = fft_ct_r2c_x<T>(phys, spec, g, nrows, nf, twx2, twx, s);
-        if (e) return e;
-        if (ctx.hook) ctx.hook(ctx.hook_ctx, sizeof(T) == 8 ? "fft_x_r2c" : "fft32_x_r2c");
-        e = fft_ct_y<-1, C>(spec, spec, g, nplanes, ncol, nf, twy, s);
-        if (ctx.hook) ctx.hook(ctx.hook_ctx, sizeof(T) == 8 ? "fft_y_forward" : "fft32_y_forward");
-        return e;
+        if (ctx.use_ct) {
+            cudaError_t e = fft_ct_r2c_x(phys, spec, g, nrows, nf, twx2, twx, s);
+            if (e) return e;
+            if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_x_r2c");
+            e = fft_ct_y<-1, C>(spec, spec, g, nplanes, ncol, nf, twy, s);
+            if (ctx.hook) ctx.hook(ctx.hook_ctx, "fft_y_forward");
+            return e;
+        }
     }
     const int rx = pick_rx(g.nxh);
     dim3 gx((nrows + rx - 1) / rx, nf);
@@ -484,7 +484,7 @@ cudaError_t fft_r2c(const FftCtx& ctx, const GridDev& g, RFields phys, Fields sp
 
 cudaError_t fft_c2r32(const FftCtx& ctx, const GridDev& g, FFields spec, FRFields phys, int nf, int nplanes,
                       cudaStream_t s) {
-    if (nf > ctx.tmp_fields || nf > kMaxFields || !ctx.tmp32) return cudaErrorInvalidValue;
+    if (ctx.use_ct || nf > ctx.tmp_fields || nf > kMaxFields || !ctx.tmp32) return cudaErrorInvalidValue;
     FFields tmp{};
     for (int f = 0; f < nf; ++f) tmp.p[f] = ctx.tmp32 + (size_t)f * g.nm * g.nz;
     return c2r_impl<float>(ctx, g, spec, phys, tmp, nf, nplanes, s, ctx.tw32_ny, ctx.tw32_nx2, ctx.tw32_nx);
@@ -492,7 +492,7 @@ cudaError_t fft_c2r32(const FftCtx& ctx, const GridDev& g, FFields spec, FRField
 
 cudaError_t fft_r2c32(const FftCtx& ctx, const GridDev& g, FRFields phys, FFields spec, int nf, int nplanes,
                       cudaStream_t s, int ncol) {
-    if (nf > kMaxFields) return cudaErrorInvalidValue;
+    if (ctx.use_ct || nf > kMaxFields) return cudaErrorInvalidValue;
     return r2c_impl<float>(ctx, g, phys, spec, nf, nplanes, s, ctx.tw32_ny, ctx.tw32_nx2, ctx.tw32_nx, ncol);
 }
 

@@ -26,17 +26,15 @@ __global__ void __launch_bounds__(kThreads) k_fft_y_ct(FieldsT<C> src, FieldsT<C
     fft_y_body<N, SIGN, C>(src, dst, g, nplanes, ncol, tw, blockIdx.x, blockIdx.z, buf);
 }
 
-// c2r along x, N = nx/2: RX rows per CTA (row = plane * ny + y).  Packs the
+// c2r along x on the FP64 pipe, N = nx/2: RX rows per CTA (row = plane * ny + y).  Packs the
 // nx/2+1 inputs of a row (Re only at kx = 0, nx/2) into Z[k] =
 // (X[k] + conj(X[N-k])) + i e^{+2 pi i k/nx} (X[k] - conj(X[N-k])), runs the
 // inverse length-N transform and writes z[m] = (x[2m], x[2m+1]) / (nx ny).
-template <int N, typename T>
-__device__ __forceinline__ void c2r_x_body(const FieldsT<typename Cx<T>::type>& src, const FieldsT<T>& dst,
-                                           const GridDev& g, int nrows,
-                                           const typename Cx<T>::type* __restrict__ tw_n,
-                                           const typename Cx<T>::type* __restrict__ tw_nx, int bx, int f,
-                                           typename Cx<T>::type* buf) {
-    using C = typename Cx<T>::type;
+template <int N>
+__device__ __forceinline__ void c2r_x_body(const Fields& src, const RFields& dst, const GridDev& g, int nrows,
+                                           const double2* __restrict__ tw_n, const double2* __restrict__ tw_nx,
+                                           int bx, int f, double2* buf) {
+    using C = double2;
     constexpr int RX = per_cta(N);
     constexpr int LD = ld_of<C>(N);
     const int row0 = bx * RX;
@@ -76,7 +74,7 @@ __device__ __forceinline__ void c2r_x_body(const FieldsT<typename Cx<T>::type>& 
     }
     __syncthreads();
     ct_fft<N, 1, +1, RX, LD>(buf, tw_n);
-    const T sc = (T)g.inv_nxny;
+    const double sc = g.inv_nxny;
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
         const int t = threadIdx.x + it * kThreads;
@@ -88,25 +86,22 @@ __device__ __forceinline__ void c2r_x_body(const FieldsT<typename Cx<T>::type>& 
     }
 }
 
-template <int N, typename T>
-__global__ void __launch_bounds__(kThreads) k_c2r_x_ct(FieldsT<typename Cx<T>::type> src, FieldsT<T> dst,
-                                                       GridDev g, int nrows,
-                                                       const typename Cx<T>::type* __restrict__ tw_n,
-                                                       const typename Cx<T>::type* __restrict__ tw_nx) {
-    __shared__ typename Cx<T>::type buf[per_cta(N) * ld_of<typename Cx<T>::type>(N)];
-    c2r_x_body<N, T>(src, dst, g, nrows, tw_n, tw_nx, blockIdx.x, blockIdx.y, buf);
+template <int N>
+__global__ void __launch_bounds__(kThreads) k_c2r_x_ct(Fields src, RFields dst, GridDev g, int nrows,
+                                                       const double2* __restrict__ tw_n,
+                                                       const double2* __restrict__ tw_nx) {
+    __shared__ double2 buf[per_cta(N) * ld_of<double2>(N)];
+    c2r_x_body<N>(src, dst, g, nrows, tw_n, tw_nx, blockIdx.x, blockIdx.y, buf);
 }
 
 // r2c along x, N = nx/2: z[m] = x[2m] + i x[2m+1], forward length-N
 // transform, X[k] = E + e^{-2 pi i k/nx} O with E = (Z[k] + conj(Z[N-k]))/2,
 // O = (Z[k] - conj(Z[N-k]))/(2i), k = 0..N.
-template <int N, typename T>
-__device__ __forceinline__ void r2c_x_body(const FieldsT<T>& src, const FieldsT<typename Cx<T>::type>& dst,
-                                           const GridDev& g, int nrows,
-                                           const typename Cx<T>::type* __restrict__ tw_n,
-                                           const typename Cx<T>::type* __restrict__ tw_nx, int bx, int f,
-                                           typename Cx<T>::type* buf) {
-    using C = typename Cx<T>::type;
+template <int N>
+__device__ __forceinline__ void r2c_x_body(const RFields& src, const Fields& dst, const GridDev& g, int nrows,
+                                           const double2* __restrict__ tw_n, const double2* __restrict__ tw_nx,
+                                           int bx, int f, double2* buf) {
+    using C = double2;
     constexpr int RX = per_cta(N);
     constexpr int LD = ld_of<C>(N);
     const int row0 = bx * RX;
@@ -134,7 +129,7 @@ __device__ __forceinline__ void r2c_x_body(const FieldsT<T>& src, const FieldsT<
         if (row0 + r < nrows) {
             const C za = buf[r * LD + sw<C>(k == N ? 0 : k)];
             const C zb = buf[r * LD + sw<C>(k == 0 ? 0 : N - k)];
-            const T hf = (T)0.5;
+            const double hf = 0.5;
             const C e = mk<C>(hf * (za.x + zb.x), hf * (za.y - zb.y));
             const C o = mk<C>(hf * (za.y + zb.y), -hf * (za.x - zb.x));
             const C p = cmul(__ldg(&tw_nx[k]), o);
@@ -143,13 +138,12 @@ __device__ __forceinline__ void r2c_x_body(const FieldsT<T>& src, const FieldsT<
     }
 }
 
-template <int N, typename T>
-__global__ void __launch_bounds__(kThreads) k_r2c_x_ct(FieldsT<T> src, FieldsT<typename Cx<T>::type> dst,
-                                                       GridDev g, int nrows,
-                                                       const typename Cx<T>::type* __restrict__ tw_n,
-                                                       const typename Cx<T>::type* __restrict__ tw_nx) {
-    __shared__ typename Cx<T>::type buf[per_cta(N) * ld_of<typename Cx<T>::type>(N)];
-    r2c_x_body<N, T>(src, dst, g, nrows, tw_n, tw_nx, blockIdx.x, blockIdx.y, buf);
+template <int N>
+__global__ void __launch_bounds__(kThreads) k_r2c_x_ct(RFields src, Fields dst, GridDev g, int nrows,
+                                                       const double2* __restrict__ tw_n,
+                                                       const double2* __restrict__ tw_nx) {
+    __shared__ double2 buf[per_cta(N) * ld_of<double2>(N)];
+    r2c_x_body<N>(src, dst, g, nrows, tw_n, tw_nx, blockIdx.x, blockIdx.y, buf);
 }
 
 // ------------------------------------------------------------------ fixed-point passes
@@ -472,21 +466,20 @@ struct RsFftY {
     }
 };
 
-template <typename T>
 struct RsC2R {
-    static constexpr int kMinCtas = sizeof(T) == 8 ? 2 : 3;
+    static constexpr int kMinCtas = 2;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        using C = typename Cx<T>::type;
+        using C = double2;
         __shared__ C buf[ct_buf_max()];
         const int gx = d.gx[kRsFftC2R];
         const int f = b / gx, bx = b - f * gx;
         const C* twn = static_cast<const C*>(d.tw_nx2);
         const C* twx = static_cast<const C*>(d.tw_nx);
         switch (d.g.nxh) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        c2r_x_body<n, T>(one_field<C>(d.tmp, f), one_field<T>(d.phys, f), d.g, d.g.nz * d.g.ny, twn, twx, bx, \
-                         0, buf);                                                                              \
+#define X_CASE(n) \
+    case n: \
+        c2r_x_body<n>(one_field<C>(d.tmp, f), one_field<double>(d.phys, f), d.g, d.g.nz * d.g.ny, twn, twx, bx, \
+                         0, buf); \
         break;
             DNS3D_CT_X_LENGTHS(X_CASE)
 #undef X_CASE
@@ -494,21 +487,20 @@ struct RsC2R {
     }
 };
 
-template <typename T>
 struct RsR2C {
-    static constexpr int kMinCtas = sizeof(T) == 8 ? 3 : 4;
+    static constexpr int kMinCtas = 3;
     static __device__ __forceinline__ void run(const RunDesc& d, int b) {
-        using C = typename Cx<T>::type;
+        using C = double2;
         __shared__ C buf[ct_buf_max()];
         const int gx = d.gx[kRsFftR2C];
         const int f = b / gx, bx = b - f * gx;
         const C* twn = static_cast<const C*>(d.tw_nx2);
         const C* twx = static_cast<const C*>(d.tw_nx);
         switch (d.g.nxh) {
-#define X_CASE(n)                                                                                              \
-    case n:                                                                                                    \
-        r2c_x_body<n, T>(one_field<T>(d.phys, f), one_field<C>(d.src, f), d.g, d.g.nz * d.g.ny, twn, twx, bx, \
-                         0, buf);                                                                              \
+#define X_CASE(n) \
+    case n: \
+        r2c_x_body<n>(one_field<double>(d.phys, f), one_field<C>(d.src, f), d.g, d.g.nz * d.g.ny, twn, twx, bx, \
+                         0, buf); \
         break;
             DNS3D_CT_X_LENGTHS(X_CASE)
 #undef X_CASE
@@ -528,8 +520,8 @@ StageKernel ragged_fft_kernel(int stage, bool mixed, bool fx) {
             return mixed ? k_stage<RsFftY<+1, 0, float, double2>> : k_stage<RsFftY<+1, 0, double, double2>>;
         case kRsFftYInv:
             return mixed ? k_stage<RsFftY<+1, 3, float, float2>> : k_stage<RsFftY<+1, 3, double, double2>>;
-        case kRsFftC2R: return k_stage<RsC2R<double>>;
-        case kRsFftR2C: return k_stage<RsR2C<double>>;
+        case kRsFftC2R: return k_stage<RsC2R>;
+        case kRsFftR2C: return k_stage<RsR2C>;
         case kRsFftYFwd:
             return mixed ? k_stage<RsFftY<-1, 0, float, float2>> : k_stage<RsFftY<-1, 0, double, double2>>;
     }
@@ -547,20 +539,20 @@ void launch_y(FieldsT<C> src, FieldsT<C> dst, const GridDev& g, int nplanes, int
     k_fft_y_ct<N, SIGN, C><<<grid, kThreads, 0, s>>>(src, dst, g, nplanes, ncol, tw);
 }
 
-template <typename T, int N>
-void launch_c2r(FieldsT<typename Cx<T>::type> src, FieldsT<T> dst, const GridDev& g, int nrows, int nf,
-                const typename Cx<T>::type* tw_n, const typename Cx<T>::type* tw_nx, cudaStream_t s) {
+template <int N>
+void launch_c2r(Fields src, RFields dst, const GridDev& g, int nrows, int nf, const double2* tw_n,
+                const double2* tw_nx, cudaStream_t s) {
     constexpr int RX = per_cta(N);
     dim3 grid((nrows + RX - 1) / RX, nf);
-    k_c2r_x_ct<N, T><<<grid, kThreads, 0, s>>>(src, dst, g, nrows, tw_n, tw_nx);
+    k_c2r_x_ct<N><<<grid, kThreads, 0, s>>>(src, dst, g, nrows, tw_n, tw_nx);
 }
 
-template <typename T, int N>
-void launch_r2c(FieldsT<T> src, FieldsT<typename Cx<T>::type> dst, const GridDev& g, int nrows, int nf,
-                const typename Cx<T>::type* tw_n, const typename Cx<T>::type* tw_nx, cudaStream_t s) {
+template <int N>
+void launch_r2c(RFields src, Fields dst, const GridDev& g, int nrows, int nf, const double2* tw_n,
+                const double2* tw_nx, cudaStream_t s) {
     constexpr int RX = per_cta(N);
     dim3 grid((nrows + RX - 1) / RX, nf);
-    k_r2c_x_ct<N, T><<<grid, kThreads, 0, s>>>(src, dst, g, nrows, tw_n, tw_nx);
+    k_r2c_x_ct<N><<<grid, kThreads, 0, s>>>(src, dst, g, nrows, tw_n, tw_nx);
 }
 
 template <int SIGN, int N>
@@ -616,12 +608,11 @@ cudaError_t fft_ct_y(FieldsT<C> src, FieldsT<C> dst, const GridDev& g, int nplan
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t fft_ct_c2r_x(FieldsT<typename Cx<T>::type> src, FieldsT<T> dst, const GridDev& g, int nrows, int nf,
-                         const typename Cx<T>::type* tw_n, const typename Cx<T>::type* tw_nx, cudaStream_t s) {
+cudaError_t fft_ct_c2r_x(Fields src, RFields dst, const GridDev& g, int nrows, int nf, const double2* tw_n,
+                         const double2* tw_nx, cudaStream_t s) {
     switch (g.nxh) {
 #define X_CASE(n) \
-    case n: launch_c2r<T, n>(src, dst, g, nrows, nf, tw_n, tw_nx, s); break;
+    case n: launch_c2r<n>(src, dst, g, nrows, nf, tw_n, tw_nx, s); break;
         DNS3D_CT_X_LENGTHS(X_CASE)
 #undef X_CASE
         default: return cudaErrorInvalidValue;
@@ -629,12 +620,11 @@ cudaError_t fft_ct_c2r_x(FieldsT<typename Cx<T>::type> src, FieldsT<T> dst, cons
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t fft_ct_r2c_x(FieldsT<T> src, FieldsT<typename Cx<T>::type> dst, const GridDev& g, int nrows, int nf,
-                         const typename Cx<T>::type* tw_n, const typename Cx<T>::type* tw_nx, cudaStream_t s) {
+cudaError_t fft_ct_r2c_x(RFields src, Fields dst, const GridDev& g, int nrows, int nf, const double2* tw_n,
+                         const double2* tw_nx, cudaStream_t s) {
     switch (g.nxh) {
 #define X_CASE(n) \
-    case n: launch_r2c<T, n>(src, dst, g, nrows, nf, tw_n, tw_nx, s); break;
+    case n: launch_r2c<n>(src, dst, g, nrows, nf, tw_n, tw_nx, s); break;
         DNS3D_CT_X_LENGTHS(X_CASE)
 #undef X_CASE
         default: return cudaErrorInvalidValue;
@@ -690,14 +680,6 @@ template cudaError_t fft_ct_y<+1, double2>(Fields, Fields, const GridDev&, int, 
 template cudaError_t fft_ct_y<-1, float2>(FFields, FFields, const GridDev&, int, int, int, const float2*,
                                          cudaStream_t);
 template cudaError_t fft_ct_y<+1, float2>(FFields, FFields, const GridDev&, int, int, int, const float2*,
-                                         cudaStream_t);
-template cudaError_t fft_ct_c2r_x<double>(Fields, RFields, const GridDev&, int, int, const double2*, const double2*,
-                                          cudaStream_t);
-template cudaError_t fft_ct_c2r_x<float>(FFields, FRFields, const GridDev&, int, int, const float2*, const float2*,
-                                         cudaStream_t);
-template cudaError_t fft_ct_r2c_x<double>(RFields, Fields, const GridDev&, int, int, const double2*, const double2*,
-                                          cudaStream_t);
-template cudaError_t fft_ct_r2c_x<float>(FRFields, FFields, const GridDev&, int, int, const float2*, const float2*,
                                          cudaStream_t);
 
 }  // namespace dns3d

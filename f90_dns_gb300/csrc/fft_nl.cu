@@ -12,7 +12,7 @@
 // pass, are left only at the outer ends, and each point's products are formed
 // in integers and rounded once at 2^-60 of the product of the row maxima, in
 // place of FP64 arithmetic.  The mixed form runs the same kernel
-// in FP32 (bitwise the separate c2r, product and r2c kernels' values).
+// in FP32.
 //
 // The x kernel: one warp per field, the warp's 32 lanes hold 32 / (N/8)
 // transforms of length N = nx/2 with 8 elements each, so every pass of the
@@ -501,8 +501,7 @@ __global__ void __launch_bounds__(kXThreads, 4) k_nl_x(Fields src, const int* ec
     x_body_fx<N>(src, ecol, ecs, dst, erow, g, nrows, ncol, tw_n, tw_nx, blockIdx.x, buf, sh);
 }
 
-// The same in FP32 (the mixed form): the arithmetic of c2r_x_body, the
-// products and r2c_x_body (fft_ct.cu), value for value.
+// The same in FP32 (the mixed form), the products in FP32 arithmetic.
 template <int N>
 __device__ __forceinline__ void x_body_32(const FFields& src, const FFields& dst, const GridDev& g, int nrows,
                                           int ncol, const float2* __restrict__ tw_n,

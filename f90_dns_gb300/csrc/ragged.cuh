@@ -56,7 +56,7 @@ struct RunDesc {
     double2 *U, *V, *W, *P, *GP, *US, *VS, *WS, *PHI, *PHIZ;
     void* spec[6];   // inverse transform inputs: u, v, w (FP64), ox, oy, oz spectra (FP32 or FP64)
     void* tmp[6];    // y-pass outputs
-    void* phys[6];   // physical planes; the products overwrite the first three
+    void* phys[6];   // physical planes of the FP64-pipe transforms; the products overwrite the first three
     void* src[3];    // nonlinear source spectra
     const void* tw_ny;
     const void* tw_nx2;

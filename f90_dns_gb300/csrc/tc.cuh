@@ -305,10 +305,7 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t* mbar, uint32_t parity, in
 }
 
 // TMEM loads issued back to back with one wait (tc_ld_wait) for all of them:
-// N = 2 or 4 consecutive columns of this thread's lane, no wait.
-__device__ __forceinline__ void tc_ld2_nw(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
-}
+// 4 consecutive columns of this thread's lane, no wait.
 __device__ __forceinline__ void tc_ld4_nw(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
