@@ -991,6 +991,9 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     g.inv_nxny = 1.0 / ((double)c.nx * (double)c.ny);
     g.refine = (c.precision == DNS3D_PREC_MIXED && c.poisson_refinement) ? 1 : 0;
     const int nz = c.nz;
+    // (first: the *_fits below go by the shared-memory limits it raises)
+    cudaError_t e = prepare_step_kernels(g);
+    if (e != cudaSuccess) { cuda_fail(h, e, "prepare"); return fail(DNS3D_E_CUDA); }
     // FP64 runs; DNS3D_TENSOR_CORES=0 keeps the FP64-pipe kernels
     const char* tcenv = std::getenv("DNS3D_TENSOR_CORES");
     const bool tc_on = c.precision == DNS3D_PREC_FP64 && !(tcenv && std::strcmp(tcenv, "0") == 0);
@@ -1090,13 +1093,11 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     if (cudaMallocHost(&h->h_out, (16 + 6 * (size_t)c.nz) * sizeof(double)) != cudaSuccess) return fail(DNS3D_E_OOM);
     if ((rc = dev_alloc(h, &h->d_flag, 4))) return fail(rc);
 
-    cudaError_t e;
     if ((e = fft_setup(h->fft, g)) != cudaSuccess) { cuda_fail(h, e, "fft_setup"); return fail(DNS3D_E_CUDA); }
     if (h->fft.fx && c.precision != DNS3D_PREC_MIXED &&
         ((rc = dev_alloc(h, &h->fft.ecol, (size_t)6 * nz * g.nxhp)) ||
          (rc = dev_alloc(h, &h->fft.erow, (size_t)3 * nz * c.ny))))
         return fail(rc);
-    if ((e = prepare_step_kernels(g)) != cudaSuccess) { cuda_fail(h, e, "prepare"); return fail(DNS3D_E_CUDA); }
 
     // per-mode operator inverses
     if (cudaMemsetAsync(h->d_flag, 0, 4 * sizeof(int), h->stream) != cudaSuccess) return fail(DNS3D_E_CUDA);
