@@ -33,11 +33,12 @@ if ROOT not in sys.path:
 WORKLOAD = "channel_128x128x65_re180_pi"
 
 # DRAM bytes of one launch of the dominant kernel (dram__bytes_read.sum +
-# dram__bytes_write.sum), from one `ncu --set full --clock-control none`
-# capture of that kernel on the same workload and build; --traffic overrides.
+# dram__bytes_write.sum), from one `ncu --clock-control none` capture of that
+# kernel on the same workload (profiles/step_kernels_by_grid.md); --traffic
+# overrides.
 NCU_TRAFFIC = {
     ("channel_128x128x65_re180_pi", "viscous_helmholtz"): 154.447104e6 + 16.572160e6,
-    ("channel_128x128x65_re180_pi", "viscous_helmholtz_tc"): 257.373952e6 + 18.197248e6,
+    ("channel_128x128x65_re180_pi", "viscous_helmholtz_tc"): 256.701440e6 + 17.730816e6,
 }
 
 
@@ -303,7 +304,7 @@ def run_reference(args) -> None:
 # per-launch DRAM traffic (ncu dram__bytes_read.sum + dram__bytes_write.sum)
 # and tensor-pipe activity of the tensor-core kernels, from one capture each
 NCU_TENSOR_PIPE = {
-    ("channel_128x128x65_re180_pi", "viscous_helmholtz_tc"): 12.6,
+    ("channel_128x128x65_re180_pi", "viscous_helmholtz_tc"): 14.2,
 }
 
 

@@ -294,7 +294,7 @@ cudaError_t smem_attr(K k, int bytes) {
 
 // A Q62 integer as two signed 32-bit limbs, w = w1 2^32 + w0 with |w0| < 2^31
 // (high word w1, low word w0), the operand form of the fixed-point products
-// (FxLimbs, fft_ct.cu).  w0 = -2^31, whose negation has no 32-bit form, is
+// (FxLimbs, fft_dev.cuh).  w0 = -2^31, whose negation has no 32-bit form, is
 // stored for w + 1 instead (2^-62 off).
 long long pack_limbs(long long w) {
     if ((int32_t)w == INT32_MIN) ++w;

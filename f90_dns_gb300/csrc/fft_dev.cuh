@@ -161,7 +161,7 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft3(C* v) {
     const C d = csub(v[1], v[2]);
     C m, id;
     if constexpr (is_fx<C>()) {
-        // t/2 rounded half up; sqrt(3)/2 as a Q62 constant
+        // t/2 rounded half up; sqrt(3)/2 as a Q63 constant
         m = mk<C>(v[0].x - ((t1.x + 1) >> 1), v[0].y - ((t1.y + 1) >> 1));
         const long long hx = fx_mulq(d.x, fx_const(kFxSqrt3h)), hy = fx_mulq(d.y, fx_const(kFxSqrt3h));
         id = SIGN > 0 ? mk<C>(-hy, hx) : mk<C>(hy, -hx);
@@ -204,9 +204,10 @@ __host__ __device__ constexpr int per_cta(int n) {
 // Shared-memory slot of element t of one transform.  FP32 passes insert one
 // padding slot after every 16 elements, so that a Stockham pass's writes at
 // stride R (8 for the radix-8 passes) fall in distinct banks instead of in
-// two: those passes are bound by shared-memory throughput.  The FP64 and
-// fixed-point passes (16-byte elements, bound by their arithmetic) keep the
-// plain layout, which needs fewer registers.
+// two: those passes are bound by shared-memory throughput.  The FP64 passes
+// and the fixed-point ones of host transfers and diagnostics (16-byte elements,
+// bound by their arithmetic) keep the plain layout, which needs fewer
+// registers; the nonlinear term's integer passes pad every 8 (swp<3>, fft_nl.cu).
 template <typename C> __host__ __device__ constexpr int sw(int t) {
     return std::is_same<C, float2>::value ? t + (t >> 4) : t;
 }

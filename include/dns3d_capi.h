@@ -268,17 +268,17 @@ int dns3d_flow_stats_noalloc(const double* u, const double* v, const double* w, 
  * per process.  Runs whose options allow it (the default convection scheme
  * and solver, transform lengths with compile-time kernels, fewer than 2^20
  * grid points -- larger runs fill the GPU with their own launches) advance in
- * ragged launches: each of the ten stages of a step (vorticity with the PI
- * update, four plane-transform passes, the products, viscous, pressure,
- * projection, walls) is ONE kernel launch over the mode tiles / transform
- * columns of all such runs of one precision and kernel variant (which stages
- * run their tensor-core forms), whatever their nx, ny, nz, with
+ * ragged launches: each stage of a step (PI update, vorticity, inverse y passes
+ * of the state and of the vorticity, x passes with the products, forward y pass,
+ * viscous, pressure, projection with the walls) is ONE kernel launch over the
+ * mode tiles / transform columns of all such runs of one precision and kernel
+ * variant (which stages run their tensor-core forms), whatever their nx, ny, nz, with
  * every run's arithmetic that of its own launches (bitwise the same results);
  * the mixed form adds one launch each for the FP64 mode (0,0) viscous and
  * pressure solves, beside the tiles.  Other runs are stepped by their own
  * launches beside them.  One step is one CUDA graph;
  * DNS3D_BATCH_TUNE times the stage tile widths for this set of runs when the
- * batch is created (the runs' PI states are restored afterwards).  The
+ * batch is created (the runs' states are left as they are).  The
  * handles stay owned by the caller and must outlive the batch; the batch
  * orders itself after work already queued on each run's stream, and later
  * work on those streams after the batch's steps. */
