@@ -112,16 +112,16 @@ size_t spec_elems(const dns3d_config& c) { return (size_t)(c.nx / 2 + 1) * c.ny 
 size_t phys_elems(const dns3d_config& c) { return (size_t)c.nx * c.ny * c.nz; }
 int n_unique_q(const dns3d_config& c) { return (c.ny / 2 + 1) * (c.nx / 2 + 1); }
 // k^2 values whose Helmholtz and Poisson inverses a handle builds.  The mixed form
-// solves every mode but (0,0) in the eigenbases: it builds that mode's and, for
-// the refusal of a k^2 that overflows, the largest k^2's (96x96x65: 2.2 ms and
-// 110 MB less than all).  A small k^2 can be refused too: where k^2 M is lost
-// beside S, the Poisson operator is S alone and its last pivot may be zero (it
-// is at nz = 3 from xlen = 1e9 on).  Boxes with a k^2 below 2^-33 (6e5 long),
-// 2^20 above the rounding of entries near 1, build them all.
+// solves every mode but (0,0) in the eigenbases and builds that mode's (96x96x65:
+// 2.2 ms and 110 MB less than all).  What it then does not see: where k^2 M is
+// lost beside S, the Poisson operator is S alone, its last pivot may be zero and
+// the handle refused (at nz = 3 from xlen = 1e9 on).  Boxes with a k^2 below 2^-33
+// (6e5 long), 2^20 above the rounding of entries near 1, build them all.  (A k^2
+// that overflows is not refused: its inverses come out as zeros.)
 int n_inverses(const dns3d_config& c) {
     const double kx = 2.0 * kPi / c.xlen, ky = 2.0 * kPi / c.ylen;
     const bool shortest = std::min(kx * kx, ky * ky) >= 0x1.0p-33;
-    return c.precision == DNS3D_PREC_MIXED && shortest ? 2 : n_unique_q(c);
+    return c.precision == DNS3D_PREC_MIXED && shortest ? 1 : n_unique_q(c);
 }
 
 // Device bytes of a handle, with the images of the tensor-core viscous solve
@@ -1047,9 +1047,7 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
     ops.he = nz - ops.ho;
     const size_t nz2 = (size_t)nz * nz;
     const size_t qstride = (size_t)ops.he * ops.he + (size_t)ops.ho * ops.ho;
-    const int nqi = n_inverses(c);  // q = 0 and the largest k^2, or all of them
-    const double ksq_ends[2] = {ksq.front(), ksq.back()};
-    double* d_ksq = nullptr;
+    const int nqi = n_inverses(c);
     double* dS = nullptr;
     if ((rc = dev_alloc(h, &ops.D1e, D1e.size())) || (rc = dev_alloc(h, &ops.D1o, D1o.size())) ||
         (rc = dev_alloc(h, &ops.D2e, D2e.size())) || (rc = dev_alloc(h, &ops.D2o, D2o.size())) ||
@@ -1057,7 +1055,7 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
         (rc = dev_alloc(h, &ops.wh, nz)) || (rc = dev_alloc(h, &ops.zw, nz)) ||
         (rc = dev_alloc(h, &ops.S0, nz)) || (rc = dev_alloc(h, &ops.Sn, nz)) ||
         (rc = dev_alloc(h, &ops.xw, g.nxhp)) || (rc = dev_alloc(h, &ops.yw, c.ny)) ||
-        (rc = dev_alloc(h, &ops.ksq, nq)) || (rc = dev_alloc(h, &d_ksq, 2)) || (rc = dev_alloc(h, &dS, nz2)) ||
+        (rc = dev_alloc(h, &ops.ksq, nq)) || (rc = dev_alloc(h, &dS, nz2)) ||
         (rc = dev_alloc(h, &ops.HinvF, (size_t)nqi * qstride)) ||
         (rc = dev_alloc(h, &ops.PinvF, (size_t)nqi * qstride)) || (rc = dev_alloc(h, &ops.PpinT, nz2)))
         return fail(rc);
@@ -1068,7 +1066,7 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
         {ops.wh, wh.data(), (size_t)nz * 8}, {ops.zw, h->zwts.data(), (size_t)nz * 8},
         {ops.S0, S0.data(), (size_t)nz * 8}, {ops.Sn, Sn.data(), (size_t)nz * 8},
         {ops.xw, xw.data(), (size_t)g.nxhp * 8}, {ops.yw, yw.data(), (size_t)c.ny * 8},
-        {ops.ksq, ksq.data(), (size_t)nq * 8}, {d_ksq, ksq_ends, sizeof(ksq_ends)}, {dS, S.data(), nz2 * 8}};
+        {ops.ksq, ksq.data(), (size_t)nq * 8}, {dS, S.data(), nz2 * 8}};
     for (auto& u : ups)
         if ((rc = upload(h, u.d, u.s, u.b))) return fail(rc);
     ops.S = dS;
@@ -1101,8 +1099,7 @@ int dns3d_create(const dns3d_config* cfg, dns3d_handle** out) {
 
     // per-mode operator inverses
     if (cudaMemsetAsync(h->d_flag, 0, 4 * sizeof(int), h->stream) != cudaSuccess) return fail(DNS3D_E_CUDA);
-    if ((e = build_inverses(g, dS, ops.wh, helm_f, nqi == nq ? ops.ksq : d_ksq, nqi, ops.HinvF, ops.PinvF, ops.PpinT, h->d_flag,
-                            h->stream)))
+    if ((e = build_inverses(g, dS, ops.wh, helm_f, ops.ksq, nqi, ops.HinvF, ops.PinvF, ops.PpinT, h->d_flag, h->stream)))
         return fail(DNS3D_E_CUDA);
     int info = 0;
     if (cudaMemcpyAsync(&info, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
