@@ -113,7 +113,7 @@ struct FftCtx {
     void* hook_ctx = nullptr;
 };
 // Compile-time-length plane transforms (fft_ct.cu) for ny in {16..512} and
-// nx/2 in {16..256} of the form 2^a 3^b; fft_ct_supported tells which grids.
+// nx/2 in {16..256} of the form 2^a or 3 2^a; fft_ct_supported tells which grids.
 bool fft_ct_supported(int ny, int nxh);
 template <int SIGN, typename C>
 cudaError_t fft_ct_y(FieldsT<C> src, FieldsT<C> dst, const GridDev& g, int nplanes, int ncol, int nf, const C* tw,

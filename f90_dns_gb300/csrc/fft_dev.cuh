@@ -10,7 +10,7 @@
 
 namespace dns3d {
 
-// Instantiated lengths: ny in {16..512}, nx/2 in {16..256}, 2^a 3^b.
+// Instantiated lengths: ny in {16..512}, nx/2 in {16..256}, 2^a or 3 2^a.
 #define DNS3D_CT_Y_LENGTHS(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512)
 #define DNS3D_CT_X_LENGTHS(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256)
 
